@@ -1,0 +1,194 @@
+"""What a user of this library has it do, as cases that can be timed and compared.
+
+Three kinds of case, each through the public entry points:
+
+``layer``     ``MoELayer.forward`` (or ``capture`` once and ``replay`` per step): the whole expert-parallel
+              MoE block on this rank's tokens, SiLU-gated experts or a single Linear per expert.
+``exchange``  ``PaddedAllToAll``: padded dispatch and arrival wait; with ``combine`` also the return
+              and the top-k weighted sum.
+``pipeline``  the separate ops in the reference's order: route and pack, ``custom_a2a``, ``shuffle``,
+              ``expert``, ``unshuffle``, ``padded_return``, ``weighted_gather``.
+
+All run on one GPU (an expert-parallel group of one rank); data is bf16, the only type the expert
+kernels take.  Tokens are N(0, 1), the router N(0, 1/D), expert weights N(0, 0.02), as in ``bench.py``.
+"""
+import math
+
+import torch
+
+from iris_testing_b200.config import PRESETS, MoEConfig
+from iris_testing_b200.models import MoELayer, heap_bytes_needed
+from iris_testing_b200.ops import custom_a2a, expert, shuffle, unshuffle
+from iris_testing_b200.ops.combine import padded_return, weighted_gather
+from iris_testing_b200.parallel.padded_a2a import PaddedAllToAll
+from iris_testing_b200.parallel.symm import SymmetricHeap
+from iris_testing_b200.utils import (alloc_return_buffers, alloc_shmem_buffers, gen_local_tokens, gen_local_weights,
+                                     gen_router, reset_dispatch_flags, route_and_pack, zipf_expert_bias)
+
+BF16 = torch.bfloat16
+
+
+def _layer(name, D, F, E, k, T, gated=True, graph=False, renorm=False, zipf=0.0):
+    return dict(name=name, kind="layer", D=D, F=F, E=E, k=k, T=T, gated=gated, graph=graph, renorm=renorm, zipf=zipf)
+
+
+def _preset(name, model, T, **over):
+    p = PRESETS[model]
+    return _layer(name, p["hidden_dim"], p["ffn_dim"], over.pop("E", p["num_experts"]), over.pop("k", p["topk"]), T, **over)
+
+
+def listed():
+    return [
+        # the smallest step a user runs: every launch, host call and dependent access shows
+        _preset("tiny-64", "tiny", 64),
+        # one decode step of a serving batch: each expert's weights are streamed for a few rows
+        _preset("mixtral-decode-64", "mixtral-8x7b", 64),
+        # a decode step of fine-grained experts under CUDA-graph replay, odd batch, renormalised weights
+        _preset("fine-decode-200", "fine-grained", 200, graph=True, renorm=True),
+        # mixed prefill and decode: a ragged batch between the weight-streaming and the compute-bound ends
+        _preset("mixtral-1000", "mixtral-8x7b", 1000),
+        # one short prompt
+        _preset("mixtral-2048", "mixtral-8x7b", 2048),
+        # the headline training / prefill step, four sequences of 4096
+        _preset("mixtral-16384", "mixtral-8x7b", 16384),
+        # many small experts, eight copies of every token
+        _preset("fine-16384", "fine-grained", 16384),
+        # the largest layer, with skewed routing (a router bias of Zipf exponent 1.2)
+        _preset("large-zipf-32768", "large", 32768, zipf=1.2),
+        # the reference's own expert, one Linear: dispatch, GEMM and combine in one kernel
+        _layer("linear-3000", 4096, 4096, 32, 2, 3000, gated=False),
+        # the padded all-to-all alone at the size of the published sweep's middle, there and back
+        dict(name="exchange-4096", kind="exchange", D=4096, E=8, k=2, T=4096, combine=True),
+        # the same for a short message, dispatch only
+        dict(name="dispatch-512", kind="exchange", D=4096, E=8, k=2, T=512, combine=False),
+        # the separate ops, as code written against the reference calls them (its published chart shape)
+        dict(name="pipeline-8192", kind="pipeline", D=768, F=768, E=32, k=2, T=8192),
+    ]
+
+
+def _log_int(rng, lo, hi):
+    return max(lo, min(hi, int(math.exp(rng.uniform(math.log(lo), math.log(hi + 1))))))
+
+
+def draw(rng):
+    kind = rng.choice(["layer"] * 7 + ["exchange"] * 2 + ["pipeline"])
+    if kind == "exchange":
+        return dict(kind=kind, D=rng.choice([768, 2048, 4096]), E=rng.choice([4, 8, 32]), k=rng.choice([1, 2, 4]),
+                    T=_log_int(rng, 128, 16384), combine=rng.random() < 0.5)
+    if kind == "pipeline":
+        D = rng.choice([256, 768, 2048])
+        return dict(kind=kind, D=D, F=D, E=rng.choice([4, 8, 32]), k=rng.choice([1, 2, 4]), T=_log_int(rng, 64, 16384))
+    model = rng.choice(["tiny", "mixtral-8x7b", "mixtral-8x7b", "fine-grained", "fine-grained", "large", "linear"])
+    graph, renorm = rng.random() < 0.25, rng.random() < 0.25
+    zipf = 1.2 if rng.random() < 0.25 else 0.0
+    if model == "linear":
+        D = rng.choice([768, 2048, 4096])
+        c = _layer("", D, rng.choice([D, D // 2]), rng.choice([4, 16, 32]), rng.choice([1, 2, 4]), _log_int(rng, 16, 16384),
+                   gated=False, graph=graph, renorm=renorm, zipf=zipf)
+    elif model == "fine-grained":
+        E = rng.choice([8, 16, 32, 64, 128])
+        c = _preset("", model, _log_int(rng, 1, 16384), E=E, k=rng.choice([1, 2, 4, 8]), graph=graph, renorm=renorm, zipf=zipf)
+    else:
+        top = {"tiny": 16384, "mixtral-8x7b": 20000, "large": 8192}[model]
+        c = _preset("", model, _log_int(rng, 1, top), graph=graph, renorm=renorm, zipf=zipf)
+    del c["name"]
+    return c
+
+
+def _prepare_layer(c, seed, dev):
+    cfg = MoEConfig(hidden_dim=c["D"], ffn_dim=c["F"], num_experts=c["E"], topk=c["k"], gated=c["gated"],
+                    renormalize=c["renorm"])
+    heap = SymmetricHeap(heap_bytes_needed(cfg, c["T"]) + (16 << 20))
+    layer = MoELayer(cfg, max_tokens=c["T"], heap=heap, seed=seed, router_std=None)
+    if c["zipf"]:
+        layer.router_bias = zipf_expert_bias(c["E"], c["zipf"], seed=seed, device=dev)
+    x = gen_local_tokens(1, c["T"], c["D"], BF16, dev, seed + 1, 0, "normal")
+    if c["graph"]:
+        layer.capture(c["T"])
+    return dict(case=c, heap=heap, layer=layer, x=x)
+
+
+def _routed(c, seed, dev):
+    x = gen_local_tokens(1, c["T"], c["D"], BF16, dev, seed + 1, 0, "normal")
+    router = gen_router(c["D"], c["E"], BF16, dev, seed, std=None)
+    payload, counts, dst_off, _, idx, wgt, plan = route_and_pack(x, router, c["k"], 1, c["E"])
+    cap = max(int(counts.max().item()), 1)          # cell capacity, settled once as a program does at its start
+    return x, router, payload, counts.contiguous(), dst_off, idx, wgt, plan, cap
+
+
+def _prepare_exchange(c, seed, dev):
+    _, _, payload, counts, dst_off, idx, wgt, plan, cap = _routed(c, seed, dev)
+    cells = c["E"] * cap * c["D"] * 2
+    heap = SymmetricHeap(cells * (2 if c["combine"] else 1) + (16 << 20))
+    a2a = PaddedAllToAll(heap, c["E"], cap, c["D"], BF16, with_return=c["combine"])
+    return dict(case=c, heap=heap, a2a=a2a, payload=payload, counts=counts, dst_off=dst_off, idx=idx, wgt=wgt, plan=plan)
+
+
+def _prepare_pipeline(c, seed, dev):
+    x, router, _, _, _, _, _, _, cap = _routed(c, seed, dev)
+    cells = c["E"] * cap * (c["D"] + c["F"]) * 2
+    heap = SymmetricHeap(cells + (16 << 20))
+    bufs = alloc_shmem_buffers(heap, 1, c["E"], cap, c["D"], BF16)
+    ret = alloc_return_buffers(heap, 1, c["E"], cap, c["F"], BF16)
+    w = gen_local_weights(c["E"], c["D"], c["F"], BF16, dev, seed, 0)
+    return dict(case=c, heap=heap, bufs=bufs, ret=ret, w=w, x=x, router=router, cap=cap)
+
+
+def prepare(case, seed):
+    dev = torch.device("cuda", torch.cuda.current_device())
+    make = {"layer": _prepare_layer, "exchange": _prepare_exchange, "pipeline": _prepare_pipeline}[case["kind"]]
+    return make(case, int(seed), dev)
+
+
+def _run_pipeline(s):
+    c, b, r = s["case"], s["bufs"], s["ret"]
+    payload, counts, dst_off, _, idx, wgt, plan = route_and_pack(s["x"], s["router"], c["k"], 1, c["E"])
+    reset_dispatch_flags(b)
+    r.ret_sync.zero_()
+    custom_a2a(payload, counts, dst_off, b.pca, b.token_buf, b.counts_ready, b.token_sync, b.heap_bases, c["E"], s["cap"])
+    packed, rows = shuffle(b.token_buf, b.pca, b.token_sync, b.counts_ready, max_rows=c["T"] * c["k"])
+    out = expert(packed, s["w"], rows)
+    padded_return(unshuffle(out, b.pca, s["cap"]), b.pca, r.ret_buf, r.ret_sync, b.heap_bases)
+    return weighted_gather(r.ret_buf, plan, idx, wgt, r.ret_sync, 1, s["cap"], status=s["heap"].status)
+
+
+def run(state):
+    c = state["case"]
+    if c["kind"] == "layer":
+        return state["layer"].replay(state["x"]) if c["graph"] else state["layer"](state["x"])
+    if c["kind"] == "pipeline":
+        return _run_pipeline(state)
+    a2a = state["a2a"]
+    a2a.dispatch(state["payload"], state["counts"], state["dst_off"])
+    a2a.wait()
+    if c["combine"]:
+        a2a.send_back()
+        return a2a.reduce(state["plan"], state["idx"], state["wgt"])
+    return a2a.token_buf, a2a.pca
+
+
+def work(case):
+    """Each input read once, each output written once; of the experts' weights those that a balanced routing uses."""
+    D, E, k, T = (case[n] for n in ("D", "E", "k", "T"))
+    if case["kind"] == "exchange":
+        rows = T * k
+        if not case["combine"]:
+            return dict(bytes=2 * rows * D * 2, flops=0)
+        return dict(bytes=rows * D * 2 + T * D * 2 + rows * 8, flops=2 * rows * D)
+    F = case["F"]
+    gated = case.get("gated", False)
+    per_expert = (3 if gated else 1) * D * F
+    used = min(E, T * k)
+    out = D if gated else F
+    return dict(bytes=T * D * 2 + D * E * 2 + used * per_expert * 2 + T * out * 2,
+                flops=2 * T * k * per_expert + 2 * T * D * E)
+
+
+def tolerance(case):
+    if case["kind"] == "exchange" and not case["combine"]:
+        return "exact"          # rows are moved, not computed
+    # Against the same path in fp64 with its bf16 roundings kept (hidden activation, weighted rows), the results are
+    # off by 1.7e-3 to 2.0e-3 relative and by at most 0.018 in one value; four times that.  With many experts per
+    # token a batch of thousands has now and then a token whose 8th and 9th logits tie to fp32 rounding, where
+    # another summation order picks the other expert: its row moves by up to its smallest weight's share.
+    return {"rel": 8e-3, "max": 0.08 if case["k"] <= 2 else 0.8}
