@@ -22,8 +22,9 @@ from iris_testing_b200.ops import custom_a2a, expert, shuffle, unshuffle
 from iris_testing_b200.ops.combine import padded_return, weighted_gather
 from iris_testing_b200.parallel.padded_a2a import PaddedAllToAll
 from iris_testing_b200.parallel.symm import SymmetricHeap
-from iris_testing_b200.utils import (alloc_return_buffers, alloc_shmem_buffers, gen_local_tokens, gen_local_weights,
-                                     gen_router, reset_dispatch_flags, route_and_pack, zipf_expert_bias)
+from iris_testing_b200.utils import (alloc_return_buffers, alloc_shmem_buffers, gen_gated_expert_weights, gen_local_tokens,
+                                     gen_local_weights, gen_router, reset_dispatch_flags, route_and_pack,
+                                     zipf_expert_bias)
 
 BF16 = torch.bfloat16
 
@@ -117,10 +118,12 @@ def _routed(c, seed, dev):
 
 
 def _prepare_exchange(c, seed, dev):
-    _, _, payload, counts, dst_off, idx, wgt, plan, cap = _routed(c, seed, dev)
+    _, _, payload, counts, dst_off, idx, wgt, plan, _ = _routed(c, seed, dev)
+    cap = min(c["T"], 3 * c["T"] * c["k"] // (2 * c["E"]) + 64)     # half as much again as a balanced routing needs
     cells = c["E"] * cap * c["D"] * 2
     heap = SymmetricHeap(cells * (2 if c["combine"] else 1) + (16 << 20))
     a2a = PaddedAllToAll(heap, c["E"], cap, c["D"], BF16, with_return=c["combine"])
+    a2a.token_buf.zero_()                           # the padding is part of what a program reads
     return dict(case=c, heap=heap, a2a=a2a, payload=payload, counts=counts, dst_off=dst_off, idx=idx, wgt=wgt, plan=plan)
 
 
@@ -165,6 +168,39 @@ def run(state):
         a2a.send_back()
         return a2a.reduce(state["plan"], state["idx"], state["wgt"])
     return a2a.token_buf, a2a.pca
+
+
+def exact(case, seed):
+    """What ``run`` returns, in fp64 and plain torch; ``None`` where rows are moved and nothing is computed."""
+    if case["kind"] == "exchange" and not case["combine"]:
+        return None
+    dev = torch.device("cuda", torch.cuda.current_device())
+    seed, D, E, k, T = int(seed), case["D"], case["E"], case["k"], case["T"]
+    f64 = torch.float64
+    layer = case["kind"] == "layer"
+    x = gen_local_tokens(1, T, D, BF16, dev, seed + 1, 0, "normal").to(f64)
+    logits = x @ gen_router(D, E, BF16, dev, seed, std=None).to(f64)
+    if layer and case["zipf"]:
+        logits += zipf_expert_bias(E, case["zipf"], seed=seed, device=dev).to(f64)
+    wgt, idx = torch.topk(torch.softmax(logits, 1), k, dim=1)
+    if layer and case["renorm"]:
+        wgt = wgt / wgt.sum(1, keepdim=True)
+    if not layer and case["kind"] == "exchange":
+        return x * wgt.sum(1, keepdim=True)      # every row comes back as it was sent
+    gated = layer and case["gated"]
+    if gated:
+        weights = gen_gated_expert_weights(E, D, case["F"], BF16, dev, seed, 0)
+    else:
+        weights = (gen_local_weights(E, D, case["F"], BF16, dev, seed, 0),)
+    y = torch.zeros(T, D if gated else case["F"], dtype=f64, device=dev)
+    for e in range(E):
+        t, s = torch.nonzero(idx == e, as_tuple=True)
+        h = x[t] @ weights[0][e].to(f64)
+        if gated:
+            h = h * torch.sigmoid(h) * (x[t] @ weights[1][e].to(f64))
+            h = h @ weights[2][e].to(f64)
+        y.index_add_(0, t, h * wgt[t, s, None])
+    return y
 
 
 def work(case):
