@@ -53,9 +53,14 @@ constexpr int STG_WARP_BYTES = 32 * STG_ROW_BYTES;    // one epilogue warp's 32 
 constexpr int STG_BYTES = 4 * STG_WARP_BYTES;         // 16 KiB
 constexpr int TMEM_COLS = 512;                        // two 256-column accumulators
 constexpr int NUM_THREADS_PLAIN = 192;
-constexpr int SENDER_WARPS = 4;    // token-sender warps per CTA in the fused-dispatch build
+constexpr int SENDER_WARPS = 8;    // token-sender warps per CTA in the fused-dispatch build
 constexpr int NUM_THREADS_FUSED = NUM_THREADS_PLAIN + SENDER_WARPS * 32;
-constexpr int SEND_ROWS = 32;   // rows per sender work unit (aligned in the destination expert's row space)
+// Rows per sender work unit (aligned in the destination expert's row space).  A unit is one CTA's
+// turn: with 32-row units a batch of a few thousand rows keeps a fraction of the CTAs copying for
+// two turns while the first M-tile waits for whole units, so short batches use 8-row units.
+constexpr int SEND_ROWS = 32;
+constexpr int SEND_ROWS_SHORT = 8;
+constexpr int SEND_SHORT_UNITS = 4;   // ... up to this many 32-row units per CTA
 
 struct __align__(16) ControlSmem {
   uint64_t full[MAX_STAGES];
@@ -210,7 +215,7 @@ __host__ __device__ __forceinline__ int received_rows(const int* cnt, int W, int
 // receive layout orders the source segments of an expert the same way (self, self-1, self-2,
 // ... modulo the world), so rows land in the order the consumer's M-tiles need them.
 __host__ __device__ __forceinline__ bool fill_bucket(ControlSmem& c, const int* cnt, int W, int EL,
-                                                     int me, int bi, int cap_rows) {
+                                                     int me, int bi, int cap_rows, int send_rows) {
   const int ET = W * EL;
   const int e = bi / W, r = bi - e * W;
   const int dst = (me + r) % W;
@@ -232,8 +237,8 @@ __host__ __device__ __forceinline__ bool fill_bucket(ControlSmem& c, const int* 
   c.b_dst_rel0[bi] = within;
   c.b_dst_mtile0[bi] = mtile0;
   c.b_dst_rank[bi] = dst;
-  // units are (bucket, aligned block of SEND_ROWS destination rows); stored un-scanned for now
-  c.b_unit_start[bi + 1] = (n > 0) ? ((within + n - 1) / SEND_ROWS - within / SEND_ROWS + 1) : 0;
+  // units are (bucket, aligned block of send_rows destination rows); stored un-scanned for now
+  c.b_unit_start[bi + 1] = (n > 0) ? ((within + n - 1) / send_rows - within / send_rows + 1) : 0;
   return !(n > 0 && group_start + within + n > cap_rows) && n >= 0;
 }
 
@@ -241,11 +246,12 @@ __host__ __device__ __forceinline__ bool fill_bucket(ControlSmem& c, const int* 
 // routing counts (`cnt` = counts_all[src][dst][e], staged in shared memory).  Runs on every
 // thread of the CTA.
 __device__ __forceinline__ void build_dispatch_tables(ControlSmem& c, const b200_dispatch_args& d,
-                                                      const int* cnt, int tid, int nthreads, WaitCtx& w) {
+                                                      const int* cnt, int tid, int nthreads, int send_rows,
+                                                      WaitCtx& w) {
   const int W = d.world, EL = d.e_local, ET = W * EL, me = d.rank;
   for (int e = tid; e < EL; e += nthreads) c.g_rows[e] = received_rows(cnt, W, EL, me, e);
   for (int bi = tid; bi < ET; bi += nthreads) {
-    if (!fill_bucket(c, cnt, W, EL, me, bi, d.cap_rows)) {
+    if (!fill_bucket(c, cnt, W, EL, me, bi, d.cap_rows, send_rows)) {
       report_status(w.status, ST_OVERFLOW);
       c.overflow = 1;
       *w.abort_flag = 1;
@@ -309,6 +315,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
   // CTA pair bookkeeping: both CTAs of a pair walk the same tile list; CTA `cta_rank`
   // owns rows [cta_rank*128, +128) of each 256-row tile and half of the weight rows.
   const uint32_t cta_rank = (CG == 2) ? cluster_ctarank() : 0u;
+  const int send_rows =
+      da.num_tokens * da.topk <= SEND_ROWS * SEND_SHORT_UNITS * static_cast<int>(gridDim.x) ? SEND_ROWS_SHORT : SEND_ROWS;
   const int sched_id = blockIdx.x / CG;
   const int sched_stride = gridDim.x / CG;
 
@@ -362,7 +370,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
       for (int i = tid; i < ncnt; i += nthreads) cnt_s[i] = __ldcg(da.counts_all + i);
     }
     __syncthreads();
-    if (!c.abort_flag) build_dispatch_tables(c, da, cnt_s, tid, nthreads, w);
+    if (!c.abort_flag) build_dispatch_tables(c, da, cnt_s, tid, nthreads, send_rows, w);
     __syncthreads();
     if (tid == 0) {
       const int ET = da.world * da.e_local;
@@ -865,10 +873,10 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
         const int j = u - c.b_unit_start[bcur];
         const int rel0 = c.b_dst_rel0[bcur];
         const int nrows = c.b_count[bcur];
-        const int blk = rel0 / SEND_ROWS + j;    // aligned row block inside the destination expert
-        const int tile = blk / (BM / SEND_ROWS); // the 128-row M-tile whose counter it feeds
-        const int p_lo = max(0, blk * SEND_ROWS - rel0);
-        const int p_hi = min(nrows, (blk + 1) * SEND_ROWS - rel0);
+        const int blk = rel0 / send_rows + j;    // aligned row block inside the destination expert
+        const int tile = blk * send_rows / BM;   // the 128-row M-tile whose counter it feeds
+        const int p_lo = max(0, blk * send_rows - rel0);
+        const int p_hi = min(nrows, (blk + 1) * send_rows - rel0);
         const int dst = c.b_dst_rank[bcur];
         const int send0 = c.b_send_start[bcur];
         const int drow0 = c.b_dst_row[bcur];
@@ -1232,7 +1240,7 @@ extern "C" int b200_debug_dispatch_tables(const int* counts_all, int world, int 
   int ok = 1;
   for (int e = 0; e < e_local; ++e) g_rows[e] = received_rows(counts_all, world, e_local, rank, e);
   for (int bi = 0; bi < ET; ++bi) {
-    if (!fill_bucket(*c, counts_all, world, e_local, rank, bi, cap_rows)) ok = 0;
+    if (!fill_bucket(*c, counts_all, world, e_local, rank, bi, cap_rows, SEND_ROWS)) ok = 0;
     tables[0 * ET + bi] = c->b_count[bi];
     tables[1 * ET + bi] = c->b_send_start[bi];
     tables[2 * ET + bi] = c->b_dst_row[bi];

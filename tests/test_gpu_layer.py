@@ -338,3 +338,16 @@ def test_layer_close_returns_its_symmetric_buffers():
     assert layer.counts_all.data_ptr() == first
     layer.close()
     heap.close()
+
+
+@pytest.mark.parametrize("T", [18944 // 2 - 1, 18944 // 2, 18944 // 2 + 1])
+def test_sender_units_on_both_sides_of_the_short_batch_line(T):
+    """Up to four 32-row units per CTA (18944 routed rows on 148 CTAs) the senders work in 8-row
+    units, above it in 32-row units: same rows at the same places either way."""
+    from iris_testing_b200.config import MoEConfig
+    from iris_testing_b200.utils import gen_local_tokens
+    cfg = MoEConfig(hidden_dim=64, ffn_dim=128, num_experts=8, topk=2)
+    layer, heap = _make(cfg, T)
+    x = gen_local_tokens(1, T, 64, torch.bfloat16, heap.device, T, 0, "normal")
+    _close(layer, x, layer(x))
+    _finish(layer)
