@@ -15,6 +15,7 @@
 #include <atomic>
 
 #include "moe_args.h"
+#include "router_mma.cuh"
 #include "sm100_ptx.cuh"
 #include "topk.cuh"
 
@@ -95,6 +96,17 @@ __global__ void router_topk_simple_kernel(const __nv_bfloat16* __restrict__ x,
   }
 }
 
+// Router of every batch the small-token path does not take (see router_mma.cuh); one tile of tokens
+// per CTA.
+template <int NT, int KS>
+__global__ void __launch_bounds__(KS * 32, KS > 8 ? 1 : 2)
+router_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wr_kmajor,
+                  const float* __restrict__ bias, int T, int D, int E, int k, int renorm,
+                  int* __restrict__ topk_idx, float* __restrict__ topk_w) {
+  extern __shared__ __align__(16) float router_smem[];
+  route_tile<NT, KS>(x, wr_kmajor, bias, T, D, E, k, renorm, -1, blockIdx.x * 16, topk_idx, topk_w, router_smem);
+}
+
 // ---------------------------------------------------------------------------
 // Plan, step 1: one CTA per expert walks the flat (token, slot) list in order
 // and gives every copy routed to that expert its stable rank in the bucket.
@@ -163,6 +175,180 @@ struct PlanPushArgs {
   unsigned long long stride_flags;
 };
 
+// Publishing this rank's counts row (see above), by every thread of one CTA in two parts: the wait for the
+// peers needs nothing of the plan and runs while that is still being built (its two dependent
+// system-scope reads took as long as the plan itself); `s_abort` is zeroed and visible before.
+__device__ __forceinline__ uint32_t push_ready(const PlanPushArgs& push, int* s_abort) {
+  uint32_t epoch = push.epoch, need = push.need_iter_done;
+  if (push.iter_ptr != nullptr) {
+    const uint32_t it = __ldcg(push.iter_ptr);
+    epoch = it + 1u;
+    need = it > 0u ? it - 1u : 0u;
+  }
+  WaitCtx w; w.abort_flag = s_abort; w.status = push.status; w.budget_ns = push.wait_budget_ns;
+  if (threadIdx.x < push.world) wait_flag_geq(push.iter_done + threadIdx.x, need, w, ST_TIMEOUT_ITER);
+  return epoch;
+}
+__device__ __forceinline__ void push_counts(const PlanPushArgs& push, uint32_t epoch, const int* counts, int E) {
+  const int tid = threadIdx.x;
+  const bool odd = push.iter_ptr != nullptr && ((epoch - 1u) & 1u);
+  const unsigned long long off_counts = odd ? push.stride_counts : 0, off_flags = odd ? push.stride_flags : 0;
+  __syncthreads();            // every peer has been seen to be ready
+  for (int p = 0; p < push.world; ++p) {
+    int* dst = reinterpret_cast<int*>(push.peer_counts[p] + off_counts) + push.rank * E;
+    for (int e = tid; e < E; e += blockDim.x) dst[e] = counts[e];
+  }
+  __syncthreads();
+  if (tid < push.world) {
+    fence_acq_rel_sys();
+    st_relaxed_sys(reinterpret_cast<uint32_t*>(push.peer_flags[tid] + off_flags) + push.rank, epoch);
+  }
+}
+
+// Stable rank of each of the warp's 32 copies (lane order) among those of the same expert that this warp
+// has seen since cnt (one entry per expert, the warp's own) was zeroed; e < 0: none.
+__device__ __forceinline__ int warp_rank(int e, int lane, int* cnt) {
+  const unsigned m = __match_any_sync(0xffffffffu, e);
+  const int pre = e >= 0 ? cnt[e] : 0;
+  __syncwarp();
+  if (e >= 0 && lane == __ffs(m) - 1) cnt[e] = pre + __popc(m);
+  __syncwarp();
+  return pre + __popc(m & ((1u << lane) - 1u));
+}
+
+// Exclusive scan of n <= 128 values (4 per lane) by one warp: start[0..n], returns nothing else.
+__device__ __forceinline__ void warp_scan_experts(const int* val, int n, int lane, int* start) {
+  int v[4], sum = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = lane * 4 + j < n ? val[lane * 4 + j] : 0;
+    sum += v[j];
+  }
+  int incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
+  }
+  int acc = incl - sum;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    if (lane * 4 + j < n) start[lane * 4 + j] = acc;
+    acc += v[j];
+  }
+  if (lane == 31) start[n] = incl;
+}
+static_assert(B200_MAX_EXPERTS <= 128, "warp_scan_experts holds four experts per lane");
+
+// ---------------------------------------------------------------------------
+// Plan with a workspace (hist, [experts][chunks] ints): the list is cut into chunks, every entry is read
+// once.  Step 1 ranks each copy inside its chunk and counts the chunk's copies per expert; step 2
+// sums the chunks before its own and places the copies.  The one-CTA-per-expert form above reads the
+// whole list once per expert twice: 26 us for 131072 copies over 64 experts, 4 MB of L2 reads per us of
+// it; this form takes 3 us plus 3 us.
+// ---------------------------------------------------------------------------
+constexpr int PLAN_THREADS = 256;
+constexpr int PLAN_SUB = 1024;       // copies per pass of a CTA
+constexpr int PLAN_MAX_CHUNKS = 148;
+
+__global__ void __launch_bounds__(PLAN_THREADS)
+plan_count_kernel(const int* __restrict__ topk_idx, int n_flat, int num_experts, int chunk,
+                  int* __restrict__ rank_in_bucket, int* __restrict__ hist) {
+  constexpr int WARPS = PLAN_THREADS / 32, PER = PLAN_SUB / PLAN_THREADS;
+  __shared__ int s_cnt[WARPS][B200_MAX_EXPERTS];
+  __shared__ int s_run[B200_MAX_EXPERTS];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int lo = blockIdx.x * chunk, hi = min(n_flat, lo + chunk);
+  for (int e = tid; e < num_experts; e += PLAN_THREADS) s_run[e] = 0;
+  for (int base = lo; base < hi; base += PLAN_SUB) {
+    for (int i = tid; i < WARPS * B200_MAX_EXPERTS; i += PLAN_THREADS) (&s_cnt[0][0])[i] = 0;
+    int ev[PER], r[PER];
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = base + (warp * PER + j) * 32 + lane;
+      ev[j] = i < hi ? topk_idx[i] : -1;
+      if (ev[j] >= num_experts) ev[j] = -1;
+      if (ev[j] < 0) ev[j] = -1;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) r[j] = warp_rank(ev[j], lane, s_cnt[warp]);
+    __syncthreads();
+    for (int e = tid; e < num_experts; e += PLAN_THREADS) {
+      int acc = s_run[e];
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) {
+        const int t = s_cnt[w][e];
+        s_cnt[w][e] = acc;
+        acc += t;
+      }
+      s_run[e] = acc;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < PER; ++j) {
+      const int i = base + (warp * PER + j) * 32 + lane;
+      if (ev[j] >= 0) rank_in_bucket[i] = s_cnt[warp][ev[j]] + r[j];
+    }
+    __syncthreads();
+  }
+  __syncthreads();
+  for (int e = tid; e < num_experts; e += PLAN_THREADS) hist[e * gridDim.x + blockIdx.x] = s_run[e];
+}
+
+__global__ void __launch_bounds__(PLAN_THREADS)
+plan_place_kernel(const int* __restrict__ topk_idx, int* __restrict__ rank_in_bucket, const int* __restrict__ hist,
+                  int n_flat, int num_experts, int chunk, int* __restrict__ counts, int* __restrict__ bucket_start,
+                  int* __restrict__ send_order, int* __restrict__ dst_slot, PlanPushArgs push, int do_push) {
+  __shared__ int s_tot[B200_MAX_EXPERTS];
+  __shared__ int s_before[B200_MAX_EXPERTS];      // copies of the expert in earlier chunks
+  __shared__ int s_start[B200_MAX_EXPERTS + 1];
+  __shared__ int s_abort;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int chunks = gridDim.x - 1, me = blockIdx.x;   // the last CTA publishes the counts meanwhile
+  uint32_t epoch = 0u;
+  if (me == chunks && do_push) {
+    if (tid == 0) s_abort = 0;
+    __syncthreads();
+    epoch = push_ready(push, &s_abort);
+  }
+  for (int e = warp; e < num_experts; e += PLAN_THREADS / 32) {
+    int before = 0, tot = 0;
+    for (int c = lane; c < chunks; c += 32) {
+      const int v = hist[e * chunks + c];
+      tot += v;
+      if (c < me) before += v;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      tot += __shfl_xor_sync(0xffffffffu, tot, o);
+      before += __shfl_xor_sync(0xffffffffu, before, o);
+    }
+    if (lane == 0) { s_tot[e] = tot; s_before[e] = before; }
+  }
+  __syncthreads();
+  if (warp == 0) warp_scan_experts(s_tot, num_experts, lane, s_start);
+  __syncthreads();
+  if (me == chunks) {
+    for (int e = tid; e <= num_experts; e += PLAN_THREADS) {
+      bucket_start[e] = s_start[e];
+      if (e < num_experts) counts[e] = s_tot[e];
+    }
+    if (do_push) push_counts(push, epoch, s_tot, num_experts);
+    return;
+  }
+  const int hi = min(n_flat, (me + 1) * chunk);
+  for (int i = me * chunk + tid; i < hi; i += PLAN_THREADS) {
+    const int e = topk_idx[i];
+    if (e < 0 || e >= num_experts) continue;
+    const int rank = s_before[e] + rank_in_bucket[i];
+    const int pos = s_start[e] + rank;
+    rank_in_bucket[i] = rank;
+    send_order[pos] = i;
+    if (dst_slot) dst_slot[i] = pos;
+  }
+}
+
 __global__ void plan_finalize_kernel(const int* __restrict__ topk_idx,
                                      const int* __restrict__ rank_in_bucket,
                                      const int* __restrict__ counts, int n_flat, int num_experts,
@@ -179,30 +365,7 @@ __global__ void plan_finalize_kernel(const int* __restrict__ topk_idx,
   __syncthreads();
   if (blockIdx.x == 0) {
     for (int e = threadIdx.x; e <= num_experts; e += blockDim.x) bucket_start[e] = s_start[e];
-    if (do_push) {
-      uint32_t epoch = push.epoch, need = push.need_iter_done;
-      unsigned long long off_counts = 0, off_flags = 0;
-      if (push.iter_ptr != nullptr) {
-        const uint32_t it = __ldcg(push.iter_ptr);
-        epoch = it + 1u;
-        need = it > 0u ? it - 1u : 0u;
-        if (it & 1u) { off_counts = push.stride_counts; off_flags = push.stride_flags; }
-      }
-      WaitCtx w; w.abort_flag = &s_abort; w.status = push.status; w.budget_ns = push.wait_budget_ns;
-      if (threadIdx.x < push.world)
-        wait_flag_geq(push.iter_done + threadIdx.x, need, w, ST_TIMEOUT_ITER);
-      __syncthreads();
-      for (int p = 0; p < push.world; ++p) {
-        int* dst = reinterpret_cast<int*>(push.peer_counts[p] + off_counts) + push.rank * num_experts;
-        for (int e = threadIdx.x; e < num_experts; e += blockDim.x) dst[e] = counts[e];
-      }
-      __syncthreads();
-      if (threadIdx.x < push.world) {
-        fence_acq_rel_sys();
-        st_release_sys(reinterpret_cast<uint32_t*>(push.peer_flags[threadIdx.x] + off_flags) + push.rank,
-                       epoch);
-      }
-    }
+    if (do_push) push_counts(push, push_ready(push, &s_abort), counts, num_experts);
   }
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_flat; i += gridDim.x * blockDim.x) {
     const int e = topk_idx[i];
@@ -215,127 +378,36 @@ __global__ void plan_finalize_kernel(const int* __restrict__ topk_idx,
 
 // ---------------------------------------------------------------------------
 // Small-token path: router AND plan in ONE launch (instead of three launches).
-// For a few thousand routed copies the layer is launch- and latency-bound, and the router GEMM on
-// tensor cores (TMEM allocation, barriers, 148 CTAs) costs more than the arithmetic.  Here one to
-// eight warps per token form the logits with 16-byte loads from the K-major router weights (the
-// tokens spread over up to 148 CTAs, so that the cold loads of a wide hidden dimension run in
-// parallel), the same softmax / top-k code picks the experts, and the CTA that
-// finishes LAST (a ticket in global memory; nobody waits) builds the plan in shared memory
-// (stable ranks per expert by ballot, scan, send order) and pushes the counts to the peers.
+// A few thousand routed copies are launch- and latency-bound.  The CTAs route one tile of tokens each
+// (router_mma.cuh: 16 tokens, the row split over the warps), and the CTA that finishes LAST (a ticket in
+// global memory; nobody waits) builds the plan in shared memory (stable ranks per expert, scan, send order)
+// and pushes the counts to the peers.
 // Limits (checked by the launcher): n_flat <= SMALL_MAX_FLAT, experts <= B200_MAX_EXPERTS.
 // ---------------------------------------------------------------------------
 constexpr int SMALL_MAX_FLAT = 4096;
-constexpr int SMALL_THREADS = 256;
-constexpr int SMALL_EG = 8;            // experts per pass over a token's row
 
-__global__ void __launch_bounds__(SMALL_THREADS)
+template <int NT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
 route_plan_small_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wr_kmajor,
                         const float* __restrict__ bias, int T, int D, int E, int k, int renorm,
                         int* __restrict__ topk_idx, float* __restrict__ topk_w, int* __restrict__ counts,
                         int* __restrict__ bucket_start, int* __restrict__ send_order,
-                        int* __restrict__ dst_slot, PlanPushArgs push, int do_push, unsigned int* ticket,
-                        int wpt) {
-  __shared__ float s_lg[SMALL_THREADS / 32][B200_MAX_EXPERTS];
-  __shared__ short s_idx[SMALL_MAX_FLAT];
-  __shared__ short s_rank[SMALL_MAX_FLAT];
-  __shared__ int s_cnt[B200_MAX_EXPERTS];
+                        int* __restrict__ dst_slot, PlanPushArgs push, int do_push, unsigned int* ticket) {
+  constexpr int THREADS = WARPS * 32;
+  constexpr int SEG = SMALL_MAX_FLAT / WARPS;      // most copies of one warp's segment
+  extern __shared__ __align__(16) float router_smem[];
+  __shared__ int s_cnt[WARPS][B200_MAX_EXPERTS];
+  __shared__ int s_tot[B200_MAX_EXPERTS];
   __shared__ int s_start[B200_MAX_EXPERTS + 1];
   __shared__ int s_abort;
   __shared__ int s_last;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nwarps = blockDim.x >> 5;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int n_flat = T * k;
   if (tid == 0) s_abort = 0;
-  // ---- router: `wpt` warps per token (a power of two up to the warps of the CTA; the host picks
-  // it so that a small batch still fills the SMs).  Each warp of a token takes every wpt-th group
-  // of 32 sixteen-byte pieces of the row, the partial logits meet in shared memory and the
-  // token's first warp does softmax and top-k.
-  const int d16 = D / 8;
-  const int tpc = nwarps / wpt;                       // tokens per CTA and pass
-  const int sub = warp % wpt, slot = warp / wpt;
-  for (int base = blockIdx.x * tpc; base < T; base += gridDim.x * tpc) {   // uniform per CTA
-    const int t = base + slot;
-    const bool tv = t < T;
-    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(tv ? t : 0) * D);
-    // Experts in groups of eight with independent accumulators, two 16-byte pieces of the row per
-    // trip: 18 (cold) loads are in flight together instead of one dependent pair at a time.
-    for (int e0 = 0; e0 < E; e0 += SMALL_EG) {
-      float acc[SMALL_EG];
-#pragma unroll
-      for (int j = 0; j < SMALL_EG; ++j) acc[j] = 0.f;
-      if (tv) {
-#pragma unroll 2
-        for (int i = lane + 32 * sub; i < d16; i += 32 * wpt) {
-          const uint4 xv = __ldg(xr + i);
-          uint4 wv[SMALL_EG];
-#pragma unroll
-          for (int j = 0; j < SMALL_EG; ++j)
-            wv[j] = __ldg(reinterpret_cast<const uint4*>(wr_kmajor + static_cast<size_t>(min(e0 + j, E - 1)) * D) + i);
-          const __nv_bfloat162* xa = reinterpret_cast<const __nv_bfloat162*>(&xv);
-#pragma unroll
-          for (int j = 0; j < SMALL_EG; ++j) {
-            const __nv_bfloat162* wa = reinterpret_cast<const __nv_bfloat162*>(&wv[j]);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const float2 a = __bfloat1622float2(xa[q]), b = __bfloat1622float2(wa[q]);
-              acc[j] = fmaf(a.x, b.x, acc[j]);
-              acc[j] = fmaf(a.y, b.y, acc[j]);
-            }
-          }
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < SMALL_EG; ++j) {
-        float a = acc[j];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
-        if (lane == 0 && e0 + j < E) s_lg[warp][e0 + j] = a;
-      }
-    }
-    __syncthreads();                                  // every warp's partial logits are in place
-    if (tv && sub == 0) {
-      float* lg = s_lg[warp];
-      for (int e = lane; e < E; e += 32) {
-        float v = bias ? bias[e] : 0.f;
-        for (int s2 = 0; s2 < wpt; ++s2) v += s_lg[warp + s2][e];
-        lg[e] = v;
-      }
-      __syncwarp();
-      float mx = -INFINITY;
-      for (int e = lane; e < E; e += 32) mx = fmaxf(mx, lg[e]);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      float sum = 0.f;
-      for (int e = lane; e < E; e += 32) sum += __expf(lg[e] - mx);
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-      TopK tk; tk.init();
-      for (int e = lane; e < E; e += 32) tk.push(lg[e], e);
-      float wsum = 0.f, my_w = 0.f;
-      int my_i = 0;
-      for (int r = 0; r < k; ++r) {
-        float bv = tk.v[0]; int bi = tk.i[0] < 0 ? 0x7fffffff : tk.i[0];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-          const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
-          const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-          if (ov > bv || (ov == bv && oi < bi)) { bv = ov; bi = oi; }
-        }
-        if (tk.i[0] == bi) {   // the winning lane pops its head
-#pragma unroll
-          for (int j = 0; j < ROUTER_MAX_K - 1; ++j) { tk.v[j] = tk.v[j + 1]; tk.i[j] = tk.i[j + 1]; }
-          tk.v[ROUTER_MAX_K - 1] = -INFINITY; tk.i[ROUTER_MAX_K - 1] = -1;
-        }
-        const float p = __expf(bv - mx) / sum;
-        wsum += p;
-        if (lane == r) { my_w = p; my_i = bi; }
-      }
-      if (lane < k) {
-        topk_idx[static_cast<size_t>(t) * k + lane] = my_i;
-        topk_w[static_cast<size_t>(t) * k + lane] = renorm ? my_w / wsum : my_w;
-      }
-    }
-    __syncthreads();                                  // the partial-logit rows are reused by the next pass
-  }
+  for (int i = tid; i < WARPS * B200_MAX_EXPERTS; i += THREADS) (&s_cnt[0][0])[i] = 0;
+  if (T > 0)
+    route_tile<NT, WARPS>(x, wr_kmajor, bias, T, D, E, k, renorm, 0x7fffffff, blockIdx.x * 16, topk_idx, topk_w,
+                             router_smem);
   // ---- hand-over: every CTA publishes its choices and takes a ticket; the last one plans
   __threadfence();
   __syncthreads();
@@ -347,61 +419,52 @@ route_plan_small_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  for (int i = tid; i < n_flat; i += blockDim.x) {
-    const int e = __ldcg(topk_idx + i);
-    s_idx[i] = static_cast<short>(min(max(e, 0), E - 1));
+  const uint32_t epoch = do_push ? push_ready(push, &s_abort) : 0u;
+  // ---- plan: stable rank of every routed copy inside its expert bucket.  Each warp ranks one
+  // contiguous segment of the list against its own counters; the counters are then scanned over the warps.
+  const int seg = ((n_flat + WARPS - 1) / WARPS + 31) & ~31;
+  const int lo = warp * seg;
+  int packed[SEG / 32];                // expert << 16 | rank inside the warp's segment
+#pragma unroll
+  for (int j = 0; j < SEG / 32; ++j) {
+    const int i = lo + j * 32 + lane;
+    packed[j] = j * 32 < seg && i < n_flat ? min(max(__ldcg(topk_idx + i), 0), E - 1) : -1;
   }
-  __syncthreads();
-  // ---- plan: stable rank of every routed copy inside its expert bucket
-  for (int e = warp; e < E; e += nwarps) {
-    int running = 0;
-    for (int base = 0; base < n_flat; base += 32) {
-      const int i = base + lane;
-      const bool hit = i < n_flat && s_idx[i] == e;
-      const unsigned b = __ballot_sync(0xffffffffu, hit);
-      if (hit) s_rank[i] = static_cast<short>(running + __popc(b & ((1u << lane) - 1u)));
-      running += __popc(b);
+#pragma unroll
+  for (int j = 0; j < SEG / 32; ++j) {
+    if (j * 32 < seg) {
+      const int r = warp_rank(packed[j], lane, s_cnt[warp]);
+      if (packed[j] >= 0) packed[j] = packed[j] << 16 | r;
     }
-    if (lane == 0) s_cnt[e] = running;
   }
   __syncthreads();
-  if (tid == 0) {
+  for (int e = tid; e < E; e += THREADS) {
     int acc = 0;
-    for (int e = 0; e < E; ++e) { s_start[e] = acc; acc += s_cnt[e]; }
-    s_start[E] = acc;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      const int t = s_cnt[w][e];
+      s_cnt[w][e] = acc;
+      acc += t;
+    }
+    s_tot[e] = acc;
   }
   __syncthreads();
-  for (int e = tid; e <= E; e += blockDim.x) {
+  if (warp == 0) warp_scan_experts(s_tot, E, lane, s_start);
+  __syncthreads();
+  for (int e = tid; e <= E; e += THREADS) {
     bucket_start[e] = s_start[e];
-    if (e < E) counts[e] = s_cnt[e];
+    if (e < E) counts[e] = s_tot[e];
   }
-  for (int i = tid; i < n_flat; i += blockDim.x) {
-    const int pos = s_start[s_idx[i]] + s_rank[i];
-    send_order[pos] = i;
-    if (dst_slot) dst_slot[i] = pos;
-  }
-  if (do_push) {     // same protocol as plan_finalize_kernel
-    uint32_t epoch = push.epoch, need = push.need_iter_done;
-    unsigned long long off_counts = 0, off_flags = 0;
-    if (push.iter_ptr != nullptr) {
-      const uint32_t it = __ldcg(push.iter_ptr);
-      epoch = it + 1u;
-      need = it > 0u ? it - 1u : 0u;
-      if (it & 1u) { off_counts = push.stride_counts; off_flags = push.stride_flags; }
-    }
-    WaitCtx w; w.abort_flag = &s_abort; w.status = push.status; w.budget_ns = push.wait_budget_ns;
-    if (tid < push.world) wait_flag_geq(push.iter_done + tid, need, w, ST_TIMEOUT_ITER);
-    __syncthreads();
-    for (int p = 0; p < push.world; ++p) {
-      int* dst = reinterpret_cast<int*>(push.peer_counts[p] + off_counts) + push.rank * E;
-      for (int e = tid; e < E; e += blockDim.x) dst[e] = s_cnt[e];
-    }
-    __syncthreads();
-    if (tid < push.world) {
-      fence_acq_rel_sys();
-      st_release_sys(reinterpret_cast<uint32_t*>(push.peer_flags[tid] + off_flags) + push.rank, epoch);
+#pragma unroll
+  for (int j = 0; j < SEG / 32; ++j) {
+    if (packed[j] >= 0) {
+      const int i = lo + j * 32 + lane, e = packed[j] >> 16;
+      const int pos = s_start[e] + s_cnt[warp][e] + (packed[j] & 0xffff);
+      send_order[pos] = i;
+      if (dst_slot) dst_slot[i] = pos;
     }
   }
+  if (do_push) push_counts(push, epoch, s_tot, E);
 }
 
 // ---------------------------------------------------------------------------
@@ -504,6 +567,62 @@ int b200_router_topk_simple(const void* x, const void* wr, const float* bias, in
   return static_cast<int>(cudaGetLastError());
 }
 
+// Tensor-core router: wr_kmajor is the router matrix as [E, D].  Returns -2 when x or wr_kmajor is not
+// 16-byte aligned.
+int b200_router_mma(const void* x, const void* wr_kmajor, const b200_router_args* ra, int T, int D, void* stream) {
+  using namespace b200;
+  if (ra == nullptr || D < 8 || D % 8 != 0 || T < 0 || ra->num_experts < 1 || ra->num_experts > 256 || ra->topk < 1 ||
+      ra->topk > ROUTER_MAX_K || ra->topk > ra->num_experts)
+    return -1;
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wr_kmajor)) & 15u) != 0) return -2;
+  if (T == 0) return 0;
+  const int E = ra->num_experts;
+  // A batch of up to 16 tokens per SM is one wave of CTAs: sixteen warps share a tile's rows and need
+  // half the dependent trips of eight.  Larger batches run two CTAs of eight warps per SM, except with
+  // more than 32 experts, where the expert rows through L1 are the limit and two CTAs gain nothing
+  // (4096 x 2048 tokens, 64 experts: 26 us with eight warps, 18 us with sixteen).
+  const bool big = T > 16 * 148;
+  auto go = [&](auto kern, int threads, int smem) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    kern<<<(T + 15) / 16, threads, smem, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(wr_kmajor), ra->bias, T, D, E,
+        ra->topk, ra->renorm, ra->topk_idx, ra->topk_w);
+    b200_count_launches(1);
+    return static_cast<int>(cudaGetLastError());
+  };
+#define B200_ROUTER(NT, KS) go(router_mma_kernel<NT, KS>, KS * 32, RouterTile<NT, KS>::smem_bytes(E))
+  if (E <= 8) return big ? B200_ROUTER(1, 8) : B200_ROUTER(1, 16);
+  if (E <= 16) return big ? B200_ROUTER(2, 8) : B200_ROUTER(2, 16);
+  if (E <= 32) return big ? B200_ROUTER(4, 8) : B200_ROUTER(4, 16);
+  return B200_ROUTER(8, 16);
+#undef B200_ROUTER
+}
+
+// Ints of workspace b200_plan_ws needs for lists of any length.
+int b200_plan_ws_ints(int num_experts) { return b200::PLAN_MAX_CHUNKS * num_experts; }
+
+// b200_plan with a workspace of b200_plan_ws_ints(num_experts) ints (contents irrelevant before and after).
+int b200_plan_ws(const int* topk_idx, int n_flat, int num_experts, int* rank_in_bucket, int* counts,
+                 int* bucket_start, int* send_order, int* dst_slot, int* workspace, const b200::PlanPushArgs* push,
+                 void* stream) {
+  using namespace b200;
+  if (num_experts < 1 || num_experts > B200_MAX_EXPERTS || n_flat < 0 || workspace == nullptr) return -1;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const long long span = static_cast<long long>(PLAN_SUB) * PLAN_MAX_CHUNKS;
+  const int chunk = PLAN_SUB * static_cast<int>(std::max(1ll, (n_flat + span - 1) / span));
+  const int chunks = std::max(1, static_cast<int>((static_cast<long long>(n_flat) + chunk - 1) / chunk));
+  plan_count_kernel<<<chunks, PLAN_THREADS, 0, st>>>(topk_idx, n_flat, num_experts, chunk, rank_in_bucket, workspace);
+  b200_count_launches(1);
+  PlanPushArgs pz;
+  memset(&pz, 0, sizeof(pz));
+  plan_place_kernel<<<chunks + 1, PLAN_THREADS, 0, st>>>(topk_idx, rank_in_bucket, workspace, n_flat, num_experts, chunk,
+                                                     counts, bucket_start, send_order, dst_slot, push ? *push : pz,
+                                                     push ? 1 : 0);
+  b200_count_launches(1);
+  return static_cast<int>(cudaGetLastError());
+}
+
 // topk_idx [n_flat] -> rank_in_bucket [n_flat], counts [E], bucket_start [E+1],
 // send_order [n_flat], dst_slot [n_flat] (optional).  `push` may be null.
 int b200_plan(const int* topk_idx, int n_flat, int num_experts, int* rank_in_bucket, int* counts,
@@ -553,20 +672,25 @@ extern "C" int b200_route_plan_small(const void* x, const void* wr_kmajor, const
       ticket == nullptr)
     return -1;
   if (static_cast<long long>(T) * k > b200::SMALL_MAX_FLAT) return -2;
+  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wr_kmajor)) & 15u) != 0) return -3;
   b200::PlanPushArgs pz;
   memset(&pz, 0, sizeof(pz));
-  const int warps = b200::SMALL_THREADS / 32;
-  // warps per token: as many as still leave every token of the batch a place on the 148 SMs
-  int wpt = warps;
-  while (wpt > 1 && static_cast<long long>(T) * wpt > 148LL * warps) wpt >>= 1;
-  const int tpc = warps / wpt;
-  const int grid = std::max(1, std::min((T + tpc - 1) / tpc, 148));
-  b200::route_plan_small_kernel<<<grid, b200::SMALL_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(wr_kmajor), bias, T, D, E, k,
-      renorm, topk_idx, topk_w, counts, bucket_start, send_order, dst_slot, push ? *push : pz, push ? 1 : 0,
-      ticket, wpt);
-  b200_count_launches(1);
-  return static_cast<int>(cudaGetLastError());
+  auto go = [&](auto kern, int threads, int smem) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    kern<<<std::max(1, (T + 15) / 16), threads, smem, static_cast<cudaStream_t>(stream)>>>(
+        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(wr_kmajor), bias, T, D, E, k, renorm,
+        topk_idx, topk_w, counts, bucket_start, send_order, dst_slot, push ? *push : pz, push ? 1 : 0, ticket);
+    b200_count_launches(1);
+    return static_cast<int>(cudaGetLastError());
+  };
+#define B200_SMALL(NT, WARPS) \
+  go(b200::route_plan_small_kernel<NT, WARPS>, WARPS * 32, b200::RouterTile<NT, WARPS>::smem_bytes(E))
+  if (E <= 8) return B200_SMALL(1, 16);
+  if (E <= 16) return B200_SMALL(2, 16);
+  if (E <= 32) return B200_SMALL(4, 16);
+  return B200_SMALL(8, 16);
+#undef B200_SMALL
 }
 
 extern "C" int b200_route_plan_small_max_flat() { return b200::SMALL_MAX_FLAT; }

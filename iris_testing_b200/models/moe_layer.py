@@ -37,7 +37,7 @@ from ..config import MoEConfig
 from ..ops import cpu_ref
 from ..ops._common import declare, ptr, stream_ptr
 from ..ops.expert import sm_count
-from ..ops.plan import Plan, PlanPushArgs, make_plan
+from ..ops.plan import Plan, PlanPushArgs, make_plan, plan_workspace
 from ..ops.router import router_kmajor, router_topk
 from ..utils import gen
 
@@ -212,6 +212,7 @@ class MoELayer(nn.Module):
         n = T * k
         self._plan = Plan(torch.empty(ET, **i32), torch.empty(ET + 1, **i32), torch.empty(n, **i32),
                           torch.empty(n, **i32), torch.empty(n, **i32))
+        self._plan_ws = plan_workspace(ET, dev)
         self._slot_reduce = declare(
             "b200_slot_reduce",
             [C.c_void_p, C.c_void_p, C.c_void_p, C.c_uint, C.c_int, C.c_int, C.c_int, C.c_void_p,
@@ -467,7 +468,7 @@ class MoELayer(nn.Module):
             idx, wgt = self.route(x)
             ev("router")
             # 2. plan (+ counts push)
-            make_plan(idx, ET, out=view, push=push)
+            make_plan(idx, ET, out=view, push=push, workspace=self._plan_ws)
             ev("plan")
 
         # 3. dispatch + GEMM1 (one kernel)

@@ -46,15 +46,21 @@ class Plan:
 
 
 def _plan_fn():
-    return declare("b200_plan", [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p,
-                                 C.c_void_p, C.c_void_p, C.POINTER(PlanPushArgs), C.c_void_p])
+    return declare("b200_plan_ws", [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p,
+                                    C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(PlanPushArgs), C.c_void_p])
+
+
+def plan_workspace(num_experts: int, device) -> torch.Tensor:
+    """Scratch of the plan kernels for lists of any length (contents irrelevant between calls; calls that
+    may overlap need separate ones)."""
+    return torch.empty(declare("b200_plan_ws_ints", [C.c_int])(num_experts), dtype=torch.int32, device=device)
 
 
 def make_plan(topk_idx: torch.Tensor, num_experts: int, out: Optional[Plan] = None,
-              push: Optional[PlanPushArgs] = None) -> Plan:
+              push: Optional[PlanPushArgs] = None, workspace: Optional[torch.Tensor] = None) -> Plan:
     """topk_idx int32 [T, k] (global expert ids) -> :class:`Plan`.
 
-    ``out`` lets a caller reuse preallocated buffers; ``push`` (fused engine only)
+    ``out`` and ``workspace`` (:func:`plan_workspace`) let a caller reuse preallocated buffers; ``push`` (fused engine only)
     makes the second kernel also publish the counts to every peer.
     """
     require(topk_idx.dtype == torch.int32, "topk_idx must be int32")
@@ -69,8 +75,9 @@ def make_plan(topk_idx: torch.Tensor, num_experts: int, out: Optional[Plan] = No
         out = Plan(torch.empty(num_experts, **i32), torch.empty(num_experts + 1, **i32),
                    torch.empty(n, **i32), torch.empty(n, **i32), torch.empty(n, **i32))
     idx = topk_idx if topk_idx.is_contiguous() else topk_idx.contiguous()
+    ws = workspace if workspace is not None else plan_workspace(num_experts, dev)
     rc = _plan_fn()(ptr(idx), n, num_experts, ptr(out.rank_in_bucket), ptr(out.counts),
-                    ptr(out.bucket_start), ptr(out.send_order), ptr(out.dst_slot),
+                    ptr(out.bucket_start), ptr(out.send_order), ptr(out.dst_slot), ptr(ws),
                     C.byref(push) if push is not None else None, stream_ptr(idx))
     if rc != 0:
         raise RuntimeError(f"plan launch failed ({rc})")

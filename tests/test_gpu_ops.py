@@ -300,3 +300,34 @@ def test_padded_all_to_all_engine_repeats_without_memsets(dev, e_local, H, T, k,
     heap.check_status()
     del a2a, probe
     heap.close()
+
+
+@pytest.mark.parametrize("T,D,E,k", [(1, 8, 1, 1), (15, 72, 8, 2), (16, 64, 9, 8), (17, 136, 16, 4), (33, 1000, 17, 2),
+                                     (31, 2048, 33, 8), (9471, 72, 8, 2), (9472, 72, 16, 2), (9473, 136, 32, 4),
+                                     (9500, 200, 65, 8), (40, 4096, 256, 8),
+                                     (4736, 64, 64, 8), (4737, 64, 64, 8)])
+def test_router_tile_edges(dev, T, D, E, k):
+    """Ragged 16-token tiles and last 64-element steps, expert passes of 8 to 64, and both sides of the
+    line to 128-token tiles (9472 tokens with 17 to 32 experts, 4736 with more)."""
+    from iris_testing_b200.ops import cpu_ref, router_topk
+    from iris_testing_b200.utils import gen_local_tokens, gen_router
+    x = gen_local_tokens(1, T, D, torch.bfloat16, dev, 1, 0, "normal")
+    wr = gen_router(D, E, torch.bfloat16, dev, 1, std=None)
+    idx, w = router_topk(x, wr, k)
+    ridx, rw = cpu_ref.router_topk_ref(x, wr, k)
+    clear = cpu_ref.clear_routing_mask(x, wr, k, None)
+    assert clear.float().mean() > 0.95
+    assert torch.equal(idx[clear], ridx[clear])
+    assert torch.allclose(w[clear], rw[clear], atol=1e-6, rtol=2e-4)      # fp32 sums of up to 4096 products
+
+
+@pytest.mark.parametrize("n,E", [(0, 4), (1, 128), (1023, 3), (1024, 128), (1025, 1), (148 * 1024, 64),
+                                 (148 * 1024 + 1, 128), (400000, 8)])
+def test_plan_chunk_edges(dev, n, E):
+    """Lists around one chunk of the plan kernels, around all chunks of one pass, and of several passes."""
+    from iris_testing_b200.ops import cpu_ref, make_plan
+    g = torch.Generator(device="cpu").manual_seed(n + E)
+    idx = torch.randint(0, E, (n, 1), generator=g, dtype=torch.int32).to(dev)
+    p, r = make_plan(idx, E), cpu_ref.plan_ref(idx, E)
+    for name in ("counts", "bucket_start", "send_order", "dst_slot", "rank_in_bucket"):
+        assert torch.equal(getattr(p, name), getattr(r, name)), name
