@@ -42,8 +42,9 @@ def route_and_pack(tokens: torch.Tensor, router: torch.Tensor, topk: int, world_
     plan: Plan = make_plan(idx, num_experts_total)
     payload = pack_rows(tokens.contiguous(), plan.send_order, topk)
     send_counts = plan.counts.view(world_size, e_local)
-    dst_sizes = send_counts.sum(dim=1).to(torch.int32)
-    dst_offsets = build_dst_offsets(send_counts)
+    starts = plan.bucket_start[::e_local].clone()       # the plan's scan, read at the destinations' first experts
+    dst_offsets = starts[:-1]
+    dst_sizes = starts[1:] - dst_offsets
     return payload, send_counts, dst_offsets, dst_sizes, idx, wgt, plan
 
 

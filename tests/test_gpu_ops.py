@@ -331,3 +331,32 @@ def test_plan_chunk_edges(dev, n, E):
     p, r = make_plan(idx, E), cpu_ref.plan_ref(idx, E)
     for name in ("counts", "bucket_start", "send_order", "dst_slot", "rank_in_bucket"):
         assert torch.equal(getattr(p, name), getattr(r, name)), name
+
+
+@pytest.mark.parametrize("G,K,N", [(1, 8, 8), (2, 64, 64), (3, 72, 200), (2, 136, 56), (32, 768, 768)])
+def test_weight_transpose_kernel(dev, G, K, N):
+    from iris_testing_b200.ops.expert import _to_kmajor_cuda as to_kmajor
+    w = torch.randn(G, K, N, device=dev).to(torch.bfloat16)
+    assert torch.equal(to_kmajor(w), w.transpose(1, 2).contiguous())
+    assert torch.equal(to_kmajor(w[:, :, : N // 2 + 1]), w[:, :, : N // 2 + 1].transpose(1, 2))   # general path
+
+
+@pytest.mark.parametrize("T,k,E,H,drop", [(1, 1, 2, 8, False), (33, 2, 4, 264, True), (100, 3, 8, 520, False),
+                                          (65, 5, 8, 2048, True), (40, 11, 16, 72, False)])
+def test_weighted_gather_row_groups(dev, T, k, E, H, drop):
+    """Rows in groups of 2, 4 and 8 (more slots than a group too), ragged last column pieces, dropped rows.
+    Sums of k products in fp32 rounded to bf16: within one bf16 step of the fp32 result."""
+    from iris_testing_b200.ops import make_plan
+    from iris_testing_b200.ops.combine import weighted_gather
+    g = torch.Generator(device="cpu").manual_seed(T + k)
+    idx = torch.stack([torch.randperm(E, generator=g)[:k] for _ in range(T)]).to(torch.int32).to(dev)
+    plan = make_plan(idx, E)
+    cap = max(int(plan.counts.max()) - (3 if drop else 0), 1)
+    ret = torch.randn(1, E, cap, H, device=dev).to(torch.bfloat16)
+    w = torch.rand(T, k, device=dev)
+    y = weighted_gather(ret, plan, idx, w, None, 1, cap)
+    m = plan.dst_slot.long() - plan.bucket_start.long()[idx.reshape(-1).long()]
+    rows = ret.reshape(-1, H).double()[idx.reshape(-1).long() * cap + m.clamp(max=cap - 1)]
+    ref = (rows * (w.reshape(-1, 1).double() * (m < cap).unsqueeze(1))).view(T, k, H).sum(1)
+    mag = (rows.abs() * w.reshape(-1, 1).double()).view(T, k, H).sum(1)
+    assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * k * 2.0 ** -23).all())
