@@ -14,6 +14,7 @@
 #include <stdint.h>
 #include <string.h>
 
+#include "launch.h"
 #include "moe_args.h"
 #include "sm100_ptx.cuh"
 
@@ -542,38 +543,52 @@ struct RetireArgs {
   unsigned long long stride_ready;   // bytes between the two parity copies of ready_counters
 };
 
+// Bound by the read of T * topk rows and the write of T; a small batch by the chain of dependent accesses, so
+// a token's row is split over `wpt` warps while SMs are idle, and whatever does not depend on the arrivals (row
+// numbers, iteration, status) is read before or along with the first look at their counter.
 template <int KMAX>   // topk <= KMAX; about eight 16-byte loads per lane are kept in flight
 __global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __restrict__ dst_slot,
                                    uint32_t* arrived, uint32_t expected, int T, int topk, int H,
                                    __nv_bfloat16* __restrict__ y, RetireArgs ra, int* status,
-                                   unsigned long long budget_ns) {
+                                   unsigned long long budget_ns, int wpt) {
   __shared__ int s_abort;
+  __shared__ uint32_t s_iter;
+  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int nwarps = (gridDim.x * blockDim.x) >> 5;
+  const int part = warp % wpt;     // this warp's share of a token's columns
+  chain_wait();
+  // results sit at the row's position in the packed send order (dst_slot), or at t*topk+s when no map is given
+  size_t row[KMAX];
+  auto find_rows = [&](int t) {
+#pragma unroll
+    for (int s = 0; s < KMAX; ++s)
+      if (s < topk)
+        row[s] = dst_slot != nullptr ? static_cast<size_t>(__ldg(dst_slot + t * topk + s))
+                                     : static_cast<size_t>(t) * topk + s;
+  };
+  if (warp / wpt < T) find_rows(warp / wpt);
+  if (threadIdx.x == 32) s_iter = ra.iter_ptr != nullptr ? __ldcg(ra.iter_ptr) : 0u;
   if (threadIdx.x == 0) {
     s_abort = 0;
     // A kernel of this step has already reported an error on this rank: its rows will never
     // arrive, so do not wait for them (the iteration is still retired below).
-    if (status != nullptr && *reinterpret_cast<volatile int*>(status) != 0) {
+    const int failed = status != nullptr ? *reinterpret_cast<volatile int*>(status) : 0;
+    const bool here = ld_acquire_sys(arrived) >= expected;
+    if (failed != 0) {
       s_abort = 1;
-    } else {
+    } else if (!here) {
       WaitCtx w; w.abort_flag = &s_abort; w.status = status; w.budget_ns = budget_ns;
       wait_flag_geq(arrived, expected, w, ST_TIMEOUT_COMBINE);
     }
   }
   __syncthreads();
   if (!s_abort) {
-    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    const int nwarps = (gridDim.x * blockDim.x) >> 5;
     constexpr int U = 8 / KMAX;    // 16-byte column chunks per lane in flight at once (times topk loads)
-    for (int t = warp; t < T; t += nwarps) {
-      // results sit at the row's position in the packed send order (dst_slot), or at
-      // t*topk+s when no map is given
-      size_t row[KMAX];
-#pragma unroll
-      for (int s = 0; s < KMAX; ++s)
-        if (s < topk)
-          row[s] = dst_slot != nullptr ? static_cast<size_t>(__ldg(dst_slot + t * topk + s))
-                                       : static_cast<size_t>(t) * topk + s;
-      for (int cb = lane * 8; cb < H; cb += 256 * U) {
+    bool first = true;
+    for (int t = warp / wpt; t < T; t += nwarps / wpt) {
+      if (!first) find_rows(t);
+      first = false;
+      for (int cb = part * 256 * U + lane * 8; cb < H; cb += 256 * U * wpt) {
         uint4 v[U][KMAX];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -610,6 +625,7 @@ __global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __
       }
     }
   }
+  chain_release();
   // retire the iteration (last block only)
   __shared__ int s_last;
   __syncthreads();
@@ -622,12 +638,10 @@ __global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __
     uint32_t done_value = ra.iter_done_value;
     uint32_t* ready = ra.ready_counters;
     if (ra.iter_ptr != nullptr) {
-      const uint32_t it = __ldcg(ra.iter_ptr);
-      done_value = it + 1u;
-      if (it & 1u) ready = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(ready) + ra.stride_ready);
+      done_value = s_iter + 1u;
+      if (s_iter & 1u) ready = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(ready) + ra.stride_ready);
     }
     for (int i = threadIdx.x; i < ra.num_ready; i += blockDim.x) ready[i] = 0u;
-    __syncthreads();
     if (threadIdx.x == 0) {
       *arrived = 0u;
       *ra.ticket = 0u;
@@ -636,7 +650,7 @@ __global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __
     __syncthreads();
     if (threadIdx.x < ra.world) {
       fence_acq_rel_sys();
-      st_release_sys(reinterpret_cast<uint32_t*>(ra.peer_iter_done[threadIdx.x]) + ra.rank, done_value);
+      st_relaxed_sys(reinterpret_cast<uint32_t*>(ra.peer_iter_done[threadIdx.x]) + ra.rank, done_value);
     }
   }
 }
@@ -846,24 +860,26 @@ int b200_slot_reduce(const void* out_slots, const int* dst_slot, void* arrived, 
                      int hidden_dim, void* y, const b200::RetireArgs* ra, int* status,
                      unsigned long long budget_ns, void* stream) {
   if (hidden_dim % 8 != 0 || ra == nullptr || topk < 1 || topk > 8) return -1;
-  int blocks = (T + 7) / 8;
+  // warps per token: up to four, while that still leaves every token a warp of its own
+  const int trip = 256 * (topk <= 2 ? 4 : topk <= 4 ? 2 : 1);      // columns of one trip of a warp
+  int wpt = 1;
+  while (wpt < 4 && wpt * trip < hidden_dim && static_cast<long long>(T) * wpt * 2 <= 148 * 4 * 8) wpt *= 2;
+  int blocks = static_cast<int>((static_cast<long long>(T) * wpt + 7) / 8);
   if (blocks < 1) blocks = 1;
   if (blocks > 148 * 4) blocks = 148 * 4;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   auto* os = static_cast<const __nv_bfloat16*>(out_slots);
   auto* ar = static_cast<uint32_t*>(arrived);
   auto* yo = static_cast<__nv_bfloat16*>(y);
-  if (topk <= 2)
-    b200::slot_reduce_kernel<2><<<blocks, 256, 0, st>>>(os, dst_slot, ar, expected, T, topk, hidden_dim, yo,
-                                                        *ra, status, budget_ns);
-  else if (topk <= 4)
-    b200::slot_reduce_kernel<4><<<blocks, 256, 0, st>>>(os, dst_slot, ar, expected, T, topk, hidden_dim, yo,
-                                                        *ra, status, budget_ns);
-  else
-    b200::slot_reduce_kernel<8><<<blocks, 256, 0, st>>>(os, dst_slot, ar, expected, T, topk, hidden_dim, yo,
-                                                        *ra, status, budget_ns);
+  auto go = [&](auto kern) {
+    return b200::launch_chained(kern, dim3(blocks), dim3(256), 0, st, os, dst_slot, ar, expected, T, topk, hidden_dim, yo,
+                                *ra, status, budget_ns, wpt);
+  };
+  const cudaError_t e = topk <= 2   ? go(b200::slot_reduce_kernel<2>)
+                        : topk <= 4 ? go(b200::slot_reduce_kernel<4>)
+                                    : go(b200::slot_reduce_kernel<8>);
   b200_count_launches(1);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(e);
 }
 
 int b200_silu_gate(const void* gate, const void* up, void* out, long long n, void* stream) {

@@ -35,6 +35,7 @@
 #include <stdio.h>
 #include <string.h>
 
+#include "launch.h"
 #include "moe_args.h"
 #include "sm100_ptx.cuh"
 #include "topk.cuh"
@@ -53,6 +54,7 @@ constexpr int STG_WARP_BYTES = 32 * STG_ROW_BYTES;    // one epilogue warp's 32 
 constexpr int STG_BYTES = 4 * STG_WARP_BYTES;         // 16 KiB
 constexpr int TMEM_COLS = 512;                        // two 256-column accumulators
 constexpr int NUM_THREADS_PLAIN = 192;
+constexpr int WEIGHT_PREFETCH = 320 << 10;   // bytes per CTA asked for ahead of the first tile (47 MB on 148 SMs)
 constexpr int SENDER_WARPS = 8;    // token-sender warps per CTA in the fused-dispatch build
 constexpr int NUM_THREADS_FUSED = NUM_THREADS_PLAIN + SENDER_WARPS * 32;
 // Rows per sender work unit (aligned in the destination expert's row space).  A unit is one CTA's
@@ -267,6 +269,82 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
                     const __grid_constant__ CUtensorMap tmap_o, const b200_gemm_args ga,
                     const b200_dispatch_args da_in, const b200_combine_args ca_in,
                     const b200_router_args ra) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
+                                             ~static_cast<uintptr_t>(1023));
+  using S = Geo<CG, NT>;
+  constexpr int STAGES = S::STAGES;
+  constexpr int STAGE_BYTES = S::STAGE_BYTES;
+  uint8_t* stage_base = smem;
+  uint8_t* staging = smem + STAGES * STAGE_BYTES;
+  ControlSmem& c = *reinterpret_cast<ControlSmem*>(staging + STG_BYTES);
+
+  const int tid = threadIdx.x;
+  const int warp = tid >> 5;
+  const int lane = tid & 31;
+  const int nthreads = blockDim.x;
+  const int G = FUSED ? da_in.e_local : ga.num_groups;
+  const int TN = (ga.N + S::TILE_N - 1) / S::TILE_N;
+  const int KB = (ga.K + BK - 1) / BK;
+  const int gm = ga.group_m > 0 ? ga.group_m : 16;
+  // CTA pair bookkeeping: both CTAs of a pair walk the same tile list; CTA `cta_rank`
+  // owns rows [cta_rank*128, +128) of each 256-row tile and half of the weight rows.
+  const uint32_t cta_rank = (CG == 2) ? cluster_ctarank() : 0u;
+  const int send_rows =
+      da_in.num_tokens * da_in.topk <= SEND_ROWS * SEND_SHORT_UNITS * static_cast<int>(gridDim.x) ? SEND_ROWS_SHORT : SEND_ROWS;
+  const int sched_id = blockIdx.x / CG;
+  const int sched_stride = gridDim.x / CG;
+
+  WaitCtx w;
+  w.abort_flag = &c.abort_flag;
+  w.status = ga.status;
+  w.budget_ns = ga.wait_budget_ns;
+
+  // ---------------------------------------------------------------- set-up
+  if (tid == 0) {
+    c.abort_flag = 0;
+    c.overflow = 0;
+    c.total_units = 0;
+    for (int i = 0; i < 64; ++i) c.ready_seen[i] = 0;
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&c.full[s], 1);
+      mbar_init(&c.empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(&c.tmem_full[a], 1);
+      mbar_init(&c.tmem_empty[a], 128 * CG);   // every epilogue thread of the pair arrives
+    }
+    mbar_init(&c.drain, 1);
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_a0);
+    if constexpr (FUSED) tma_prefetch_desc(&tmap_a1);
+    tma_prefetch_desc(&tmap_b);
+    if (ga.tma_store) tma_prefetch_desc(&tmap_o);
+  }
+  if (warp == 1) {
+    if constexpr (CG == 2) {
+      tmem_alloc_pair(&c.tmem_base, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(&c.tmem_base, TMEM_COLS);
+      tmem_relinquish();
+    }
+  }
+  if (EPI != B200_EPI_ROUTER && (ga.l2_hints & 16) && warp == 2 && lane == 0) {
+    // While the kernels before this one finish (routing, the last CTAs of the first GEMM), HBM idles: ask L2 for
+    // the first k-blocks of the weight tile this CTA will probably take first (one M-tile per group).
+    const int g = sched_id / TN, n = sched_id - g * TN;
+    const int brow = g * ga.N + n * S::TILE_N + static_cast<int>(cta_rank) * S::B_ROWS;
+    if (g < G)
+      for (int kb = 0; kb < min(KB, WEIGHT_PREFETCH / S::B_STAGE_BYTES); ++kb)
+#pragma unroll
+        for (int h = 0; h < NT; ++h) l2_prefetch_2d(&tmap_b, kb * BK, brow + h * BN);
+  }
+  __syncthreads();
+  if constexpr (CG == 2) cluster_sync_all();   // the peer's barriers exist before anyone signals them
+
+  chain_wait();    // nothing above touches what an earlier kernel wrote
+  if constexpr (EPI != B200_EPI_COMBINE) chain_release();
   // Per-parity state: the iteration number lives in device memory (when iter_ptr is set), so
   // the same launch arguments serve every iteration and a captured graph can be replayed.
   b200_dispatch_args da = da_in;
@@ -294,68 +372,6 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
       ca.row_meta = reinterpret_cast<const char*>(ca.row_meta) + ca.stride_meta;
   }
   const CUtensorMap& tmap_a = (FUSED && parity) ? tmap_a1 : tmap_a0;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~static_cast<uintptr_t>(1023));
-  using S = Geo<CG, NT>;
-  constexpr int STAGES = S::STAGES;
-  constexpr int STAGE_BYTES = S::STAGE_BYTES;
-  uint8_t* stage_base = smem;
-  uint8_t* staging = smem + STAGES * STAGE_BYTES;
-  ControlSmem& c = *reinterpret_cast<ControlSmem*>(staging + STG_BYTES);
-
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5;
-  const int lane = tid & 31;
-  const int nthreads = blockDim.x;
-  const int G = FUSED ? da.e_local : ga.num_groups;
-  const int TN = (ga.N + S::TILE_N - 1) / S::TILE_N;
-  const int KB = (ga.K + BK - 1) / BK;
-  const int gm = ga.group_m > 0 ? ga.group_m : 16;
-  // CTA pair bookkeeping: both CTAs of a pair walk the same tile list; CTA `cta_rank`
-  // owns rows [cta_rank*128, +128) of each 256-row tile and half of the weight rows.
-  const uint32_t cta_rank = (CG == 2) ? cluster_ctarank() : 0u;
-  const int send_rows =
-      da.num_tokens * da.topk <= SEND_ROWS * SEND_SHORT_UNITS * static_cast<int>(gridDim.x) ? SEND_ROWS_SHORT : SEND_ROWS;
-  const int sched_id = blockIdx.x / CG;
-  const int sched_stride = gridDim.x / CG;
-
-  WaitCtx w;
-  w.abort_flag = &c.abort_flag;
-  w.status = ga.status;
-  w.budget_ns = ga.wait_budget_ns;
-
-  // ---------------------------------------------------------------- set-up
-  if (tid == 0) {
-    c.abort_flag = 0;
-    c.overflow = 0;
-    c.total_units = 0;
-    for (int i = 0; i < 64; ++i) c.ready_seen[i] = 0;
-    for (int s = 0; s < STAGES; ++s) {
-      mbar_init(&c.full[s], 1);
-      mbar_init(&c.empty[s], 1);
-    }
-    for (int a = 0; a < 2; ++a) {
-      mbar_init(&c.tmem_full[a], 1);
-      mbar_init(&c.tmem_empty[a], 128 * CG);   // every epilogue thread of the pair arrives
-    }
-    mbar_init(&c.drain, 1);
-    fence_mbar_init();
-    tma_prefetch_desc(&tmap_a);
-    tma_prefetch_desc(&tmap_b);
-    if (ga.tma_store) tma_prefetch_desc(&tmap_o);
-  }
-  if (warp == 1) {
-    if constexpr (CG == 2) {
-      tmem_alloc_pair(&c.tmem_base, TMEM_COLS);
-      tmem_relinquish_pair();
-    } else {
-      tmem_alloc(&c.tmem_base, TMEM_COLS);
-      tmem_relinquish();
-    }
-  }
-  __syncthreads();
-  if constexpr (CG == 2) cluster_sync_all();   // the peer's barriers exist before anyone signals them
 
   if constexpr (FUSED) {
     if (da.trace != nullptr && blockIdx.x == 0 && tid == 0) da.trace[0] = globaltimer_ns();
@@ -940,6 +956,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
   // ---------------------------------------------------------------- teardown
   tc_fence_before_sync();
   __syncthreads();
+  if constexpr (EPI == B200_EPI_COMBINE) chain_release();
   if constexpr (CG == 2) cluster_sync_all();   // the leader's MMAs read both CTAs' shared memory
   if (warp == 1) {
     tc_fence_after_sync();
@@ -1007,11 +1024,12 @@ static int launch_variant(const CUtensorMap& ta, const CUtensorMap& ta1, const C
   cfg.blockDim = dim3(FUSED ? NUM_THREADS_FUSED : NUM_THREADS_PLAIN, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = CG;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1] = chained_attribute();
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   // The kernel is persistent and its CTAs wait on one another (sender work is strided over the
@@ -1028,6 +1046,7 @@ static int launch_variant(const CUtensorMap& ta, const CUtensorMap& ta1, const C
   if (resident_clusters < 1) return ERR_NOT_RESIDENT;
   if (static_cast<int>(cfg.gridDim.x) > resident_clusters * CG) cfg.gridDim.x = resident_clusters * CG;
   b200_count_launches(1);
+  cfg.numAttrs = 2;
   return static_cast<int>(cudaLaunchKernelEx(&cfg, kern, ta, ta1, tb, to, ga, da, ca, ra));
 }
 

@@ -85,7 +85,8 @@ typedef struct {
   long long a_rows;               // rows of the activation (and EPI 0/1 output) buffer: the group sizes
                                   // read on the device may not add up to more (filled by the launcher)
   int l2_hints;                   // L2 eviction priorities: 1 = keep activations (evict last), 2 = stream
-                                  // weights (evict first), 4 = stream the EPI 0/1 output; 0 = none
+                                  // weights (evict first), 4 = stream the EPI 0/1 output; 0 = none.  16: prefetch the
+                                  // first weight tiles before the kernels ahead in the stream have finished
   int tma_store;                  // EPI 0/1: full 32-row boxes leave through bulk tensor stores (set by
                                   // the launcher when the output is 16-byte aligned; -1 on entry forbids it)
   int wide_tiles;                 // CTA pairs: 1 = 512-column tiles (both accumulators per tile); 0 / -1 = off

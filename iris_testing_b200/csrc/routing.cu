@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <atomic>
 
+#include "launch.h"
 #include "moe_args.h"
 #include "router_mma.cuh"
 #include "sm100_ptx.cuh"
@@ -104,6 +105,8 @@ router_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __re
                   const float* __restrict__ bias, int T, int D, int E, int k, int renorm,
                   int* __restrict__ topk_idx, float* __restrict__ topk_w) {
   extern __shared__ __align__(16) float router_smem[];
+  chain_wait();
+  chain_release();
   route_tile<NT, KS>(x, wr_kmajor, bias, T, D, E, k, renorm, -1, blockIdx.x * 16, topk_idx, topk_w, router_smem);
 }
 
@@ -259,6 +262,8 @@ plan_count_kernel(const int* __restrict__ topk_idx, int n_flat, int num_experts,
   __shared__ int s_run[B200_MAX_EXPERTS];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int lo = blockIdx.x * chunk, hi = min(n_flat, lo + chunk);
+  chain_wait();
+  chain_release();
   for (int e = tid; e < num_experts; e += PLAN_THREADS) s_run[e] = 0;
   for (int base = lo; base < hi; base += PLAN_SUB) {
     for (int i = tid; i < WARPS * B200_MAX_EXPERTS; i += PLAN_THREADS) (&s_cnt[0][0])[i] = 0;
@@ -307,6 +312,8 @@ plan_place_kernel(const int* __restrict__ topk_idx, int* __restrict__ rank_in_bu
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int chunks = gridDim.x - 1, me = blockIdx.x;   // the last CTA publishes the counts meanwhile
   uint32_t epoch = 0u;
+  chain_wait();
+  chain_release();
   if (me == chunks && do_push) {
     if (tid == 0) s_abort = 0;
     __syncthreads();
@@ -405,6 +412,8 @@ route_plan_small_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   const int n_flat = T * k;
   if (tid == 0) s_abort = 0;
   for (int i = tid; i < WARPS * B200_MAX_EXPERTS; i += THREADS) (&s_cnt[0][0])[i] = 0;
+  chain_wait();
+  chain_release();
   if (T > 0)
     route_tile<NT, WARPS>(x, wr_kmajor, bias, T, D, E, k, renorm, 0x7fffffff, blockIdx.x * 16, topk_idx, topk_w,
                              router_smem);
@@ -585,11 +594,11 @@ int b200_router_mma(const void* x, const void* wr_kmajor, const b200_router_args
   auto go = [&](auto kern, int threads, int smem) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
-    kern<<<(T + 15) / 16, threads, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(wr_kmajor), ra->bias, T, D, E,
-        ra->topk, ra->renorm, ra->topk_idx, ra->topk_w);
+    e = launch_chained(kern, dim3((T + 15) / 16), dim3(threads), smem, static_cast<cudaStream_t>(stream),
+                       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(wr_kmajor), ra->bias, T,
+                       D, E, ra->topk, ra->renorm, ra->topk_idx, ra->topk_w);
     b200_count_launches(1);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(e);
   };
 #define B200_ROUTER(NT, KS) go(router_mma_kernel<NT, KS>, KS * 32, RouterTile<NT, KS>::smem_bytes(E))
   if (E <= 8) return big ? B200_ROUTER(1, 8) : B200_ROUTER(1, 16);
@@ -612,15 +621,17 @@ int b200_plan_ws(const int* topk_idx, int n_flat, int num_experts, int* rank_in_
   const long long span = static_cast<long long>(PLAN_SUB) * PLAN_MAX_CHUNKS;
   const int chunk = PLAN_SUB * static_cast<int>(std::max(1ll, (n_flat + span - 1) / span));
   const int chunks = std::max(1, static_cast<int>((static_cast<long long>(n_flat) + chunk - 1) / chunk));
-  plan_count_kernel<<<chunks, PLAN_THREADS, 0, st>>>(topk_idx, n_flat, num_experts, chunk, rank_in_bucket, workspace);
+  cudaError_t e = launch_chained(plan_count_kernel, dim3(chunks), dim3(PLAN_THREADS), 0, st, topk_idx, n_flat,
+                                 num_experts, chunk, rank_in_bucket, workspace);
   b200_count_launches(1);
+  if (e != cudaSuccess) return static_cast<int>(e);
   PlanPushArgs pz;
   memset(&pz, 0, sizeof(pz));
-  plan_place_kernel<<<chunks + 1, PLAN_THREADS, 0, st>>>(topk_idx, rank_in_bucket, workspace, n_flat, num_experts, chunk,
-                                                     counts, bucket_start, send_order, dst_slot, push ? *push : pz,
-                                                     push ? 1 : 0);
+  e = launch_chained(plan_place_kernel, dim3(chunks + 1), dim3(PLAN_THREADS), 0, st, topk_idx, rank_in_bucket, workspace,
+                     n_flat, num_experts, chunk, counts, bucket_start, send_order, dst_slot, push ? *push : pz,
+                     push ? 1 : 0);
   b200_count_launches(1);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(e);
 }
 
 // topk_idx [n_flat] -> rank_in_bucket [n_flat], counts [E], bucket_start [E+1],
@@ -678,11 +689,12 @@ extern "C" int b200_route_plan_small(const void* x, const void* wr_kmajor, const
   auto go = [&](auto kern, int threads, int smem) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return static_cast<int>(e);
-    kern<<<std::max(1, (T + 15) / 16), threads, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(wr_kmajor), bias, T, D, E, k, renorm,
-        topk_idx, topk_w, counts, bucket_start, send_order, dst_slot, push ? *push : pz, push ? 1 : 0, ticket);
+    e = b200::launch_chained(kern, dim3(std::max(1, (T + 15) / 16)), dim3(threads), smem,
+                             static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x),
+                             static_cast<const __nv_bfloat16*>(wr_kmajor), bias, T, D, E, k, renorm, topk_idx, topk_w,
+                             counts, bucket_start, send_order, dst_slot, push ? *push : pz, push ? 1 : 0, ticket);
     b200_count_launches(1);
-    return static_cast<int>(cudaGetLastError());
+    return static_cast<int>(e);
   };
 #define B200_SMALL(NT, WARPS) \
   go(b200::route_plan_small_kernel<NT, WARPS>, WARPS * 32, b200::RouterTile<NT, WARPS>::smem_bytes(E))

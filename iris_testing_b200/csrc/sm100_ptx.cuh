@@ -207,6 +207,20 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, WaitCt
 }
 
 // ----------------------------------------------------------------------------
+// Programmatic dependent launch.  A kernel launched with launch_chained (launch.h) may start while its
+// predecessor in the stream still runs: before chain_wait() it touches nothing that an earlier kernel
+// writes or reads (its own set-up, and prefetches of weights into L2, which is where memory is coherent);
+// chain_wait() returns when the predecessor has completed and its writes are visible, and with it, since
+// every kernel waits for its own predecessor, everything before.  chain_release() lets the next kernel's CTAs
+// start wherever there is room: at once where that kernel runs one CTA per SM or only a few CTAs, at the
+// end where it is a grid of many small CTAs, which would pile up on the first SMs to come free (24 us
+// instead of 18 us for the slot reduction of 3000 tokens).  Both are no-ops in a kernel that was
+// launched the ordinary way.
+// ----------------------------------------------------------------------------
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ----------------------------------------------------------------------------
 // TMA: tiled 2-D load global -> shared (this CTA only; never multicast).
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, uint64_t* bar, int x,
@@ -299,6 +313,10 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // (16-byte aligned); no data reaches the SM.
 __device__ __forceinline__ void l2_prefetch_bulk(const void* p, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// Asks L2 to fetch one box of a tensor map (x as for a load).
+__device__ __forceinline__ void l2_prefetch_2d(const void* tmap, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
 }
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");

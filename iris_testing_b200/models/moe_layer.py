@@ -513,7 +513,9 @@ class MoELayer(nn.Module):
         ga.num_groups, ga.K, ga.group_m = EL, D, self.group_m[0]
         ga.status, ga.wait_budget_ns = status_p, self._budget_ns
         ga.cta_pair = self._cta_pair
-        ga.l2_hints = self.l2_hints[0]
+        # a prefetch ahead of the routing pays when every expert will be read
+        prefetch = 16 if T * k >= 4 * ET else 0
+        ga.l2_hints = self.l2_hints[0] | prefetch
         ga.tma_store = 0 if self.tma_store else -1
         ga.wide_tiles = self.wide_tiles[0]
         recv = self.recv[0]
@@ -531,7 +533,7 @@ class MoELayer(nn.Module):
             gb.group_rows = self.group_rows.data_ptr()
             gb.status, gb.wait_budget_ns = status_p, self._budget_ns
             gb.cta_pair = self._cta_pair
-            gb.l2_hints = self.l2_hints[1]
+            gb.l2_hints = self.l2_hints[1] | prefetch
             gb.wide_tiles = self.wide_tiles[1]
             nv.check(lib.b200_grouped_gemm(ptr(self.hidden), self.cap_rows, ptr(self.w2), nv.EPI_COMBINE,
                                            0, C.byref(gb), None, C.byref(ca), None, self._ctas, st),

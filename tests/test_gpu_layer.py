@@ -351,3 +351,19 @@ def test_sender_units_on_both_sides_of_the_short_batch_line(T):
     x = gen_local_tokens(1, T, 64, torch.bfloat16, heap.device, T, 0, "normal")
     _close(layer, x, layer(x))
     _finish(layer)
+
+
+@pytest.mark.parametrize("D,k,T", [(8, 1, 1), (1024, 2, 37), (1032, 2, 300), (4096, 2, 592), (4096, 2, 593),
+                                   (2048, 8, 1184), (520, 4, 2368), (2048, 3, 2400)])
+def test_slot_reduction_splits_rows_over_warps(D, k, T):
+    """One, two and four warps per token in the slot reduction, ragged column pieces, and the next step's
+    kernels started early: ten steps in a row without a synchronisation, every one checked."""
+    from iris_testing_b200.config import MoEConfig
+    from iris_testing_b200.utils import gen_local_tokens
+    cfg = MoEConfig(hidden_dim=D, ffn_dim=128, num_experts=8, topk=k)
+    layer, heap = _make(cfg, T)
+    xs = [gen_local_tokens(1, T, D, torch.bfloat16, heap.device, i, 0, "normal") for i in range(10)]
+    ys = [layer(x) for x in xs]
+    for x, y in zip(xs, ys):
+        _close(layer, x, y)
+    _finish(layer)
