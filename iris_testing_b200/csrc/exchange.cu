@@ -362,9 +362,10 @@ __global__ void padded_wait_kernel(const int* pca, const uint32_t* counts_ready,
 // that copy; bucket_start / send_counts locate its (dst, e, m) cell.
 // Waits (bounded) until every expert rank has returned its tiles.
 // Bound by the read of T*k rows and the write of T: a warp finds its token's rows and weights once and keeps
-// about eight 16-byte loads per lane in flight (with one column piece at a time behind the three dependent
-// index reads, 4096 x 4096 with k = 2 took 30 us, 3.3 TB/s).
-template <int KMAX>   // rows gathered at a time; any topk
+// U x KMAX 16-byte loads per lane in flight.  Wide rows take eight of them (4096 x 4096 with k = 2: 18 us; one
+// column piece at a time behind the three dependent index reads: 27 us); rows of up to 1024 columns end before
+// that pays, and more warps on the SM hide the index reads better.
+template <int KMAX, int U>   // KMAX: rows gathered at a time (any topk); U: 16-byte column pieces per lane
 __global__ void __launch_bounds__(256)
 weighted_gather_kernel(const __nv_bfloat16* __restrict__ ret_buf,
                        const int* __restrict__ dst_slot,
@@ -389,7 +390,6 @@ weighted_gather_kernel(const __nv_bfloat16* __restrict__ ret_buf,
   __syncthreads();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  constexpr int U = 8 / KMAX;      // 16-byte column pieces per lane in flight (times KMAX rows)
   for (int t = warp; t < T && !s_abort; t += nwarps) {
     const uint4* row[KMAX];        // null: no such slot, or dropped by capacity
     float wv[KMAX];
@@ -835,9 +835,11 @@ int b200_weighted_gather(const void* ret_buf, const int* dst_slot, const int* to
         static_cast<uint32_t*>(ret_sync), send_counts, T, topk, world, e_local, cap, hidden_dim,
         block_m, static_cast<__nv_bfloat16*>(y), status, budget_ns, ticket);
   };
-  if (topk <= 2) go(b200::weighted_gather_kernel<2>);
-  else if (topk <= 4) go(b200::weighted_gather_kernel<4>);
-  else go(b200::weighted_gather_kernel<8>);
+  const bool wide = hidden_dim > 1024;
+  if (topk == 1) wide ? go(b200::weighted_gather_kernel<1, 4>) : go(b200::weighted_gather_kernel<1, 1>);
+  else if (topk == 2) wide ? go(b200::weighted_gather_kernel<2, 4>) : go(b200::weighted_gather_kernel<2, 1>);
+  else if (topk <= 4) wide ? go(b200::weighted_gather_kernel<4, 2>) : go(b200::weighted_gather_kernel<4, 1>);
+  else go(b200::weighted_gather_kernel<8, 1>);
   b200_count_launches(1);
   return static_cast<int>(cudaGetLastError());
 }
