@@ -282,6 +282,7 @@ class MoELayer(nn.Module):
                        if cfg.gated else None)
         self._trace = None
         self._graph = None
+        self._prepare_launches()
 
     def memory_bytes(self) -> dict:
         """Bytes this layer holds per rank: symmetric (peer-visible) and local buffers, weights apart."""
@@ -427,16 +428,98 @@ class MoELayer(nn.Module):
             raise ValueError(f"x must be [T <= {self.max_tokens}, {D}]")
         if x.dtype != cfg.dtype or not x.is_contiguous():
             x = x.to(cfg.dtype).contiguous()
-        lib = nv.lib()
-        iter_p = self.iter_dev.data_ptr()
-        esz = 2   # bytes per bf16
         st = stream_ptr(x)
-        status_p = heap.status.data_ptr()
-
-        ev = self._mark if self.profile else (lambda name: None)
-        if self.profile:
+        ev = self._mark if self.profile else None
+        if ev:
             self.phase_events = []
-        ev("start")
+            ev("start")
+        plan = self._plan
+        n = T * k
+        if self.uses_small_path(T):
+            # 1+2. small batch: router and plan in one launch
+            idx = torch.empty((T, k), dtype=torch.int32, device=x.device)
+            wgt = torch.empty((T, k), dtype=torch.float32, device=x.device)
+            bias = None if self.router_bias is None else self.router_bias.to(
+                device=x.device, dtype=torch.float32).contiguous()
+            nv.check(self._route_plan_small(x.data_ptr(), router_kmajor(self.router).data_ptr(), ptr(bias), T, D, ET, k,
+                                            int(cfg.renormalize), idx.data_ptr(), wgt.data_ptr(),
+                                            *self._plan_ptrs, self._push_p, self._small_ticket.data_ptr(), st),
+                     "route+plan launch")
+            if ev:
+                ev("router")
+                ev("plan")
+        else:
+            # 1. router
+            idx, wgt = self.route(x)
+            if ev:
+                ev("router")
+            # 2. plan (+ counts push)
+            view = Plan(plan.counts, plan.bucket_start, plan.send_order[:n], plan.dst_slot[:n],
+                        plan.rank_in_bucket[:n])
+            make_plan(idx, ET, out=view, push=self._push, workspace=self._plan_ws)
+            if ev:
+                ev("plan")
+
+        # 3. dispatch + GEMM1 (one kernel); per-call fields go into copies of the prepared blocks
+        da = nv.DispatchArgs.from_buffer_copy(self._da)
+        da.num_tokens, da.topk = T, k
+        da.x = x.data_ptr()
+        da.topk_weight = wgt.data_ptr()
+        da.drop_signal = int(self.drop_signal)
+        if self.trace_arrivals:
+            if self._trace is None:
+                self._trace = torch.zeros(2 + 2 * self.cap_mtiles, dtype=torch.int64, device=x.device)
+            self._trace.zero_()
+            da.trace = self._trace.data_ptr()
+            da.trace_tiles = self.cap_mtiles
+        # a prefetch ahead of the routing pays when every expert will be read
+        prefetch = 16 if T * k >= 4 * ET else 0
+        ga = nv.GemmArgs.from_buffer_copy(self._ga)
+        ga.group_m = self.group_m[0]
+        ga.l2_hints = self.l2_hints[0] | prefetch
+        ga.tma_store = 0 if self.tma_store else -1
+        ga.wide_tiles = self.wide_tiles[0]
+        gemm = self._gemm
+        if cfg.gated:
+            nv.check(gemm(self._recv_p, self.cap_rows, self.w13.data_ptr(), nv.EPI_SILU_GATE, 1, C.byref(ga), C.byref(da),
+                          None, None, self._ctas, st), "dispatch+GEMM1 launch")
+            if ev:
+                ev("dispatch+gemm1")
+            # 4. GEMM2 + combine (one kernel)
+            gb = nv.GemmArgs.from_buffer_copy(self._gb)
+            gb.group_m = self.group_m[1]
+            gb.l2_hints = self.l2_hints[1] | prefetch
+            gb.wide_tiles = self.wide_tiles[1]
+            nv.check(gemm(self.hidden.data_ptr(), self.cap_rows, self.w2.data_ptr(), nv.EPI_COMBINE, 0, C.byref(gb), None,
+                          self._ca_p, None, self._ctas, st), "GEMM2+combine launch")
+            if ev:
+                ev("gemm2+combine")
+        else:
+            # single Linear: dispatch, GEMM and combine are ONE kernel
+            nv.check(gemm(self._recv_p, self.cap_rows, self.w13.data_ptr(), nv.EPI_COMBINE, 1, C.byref(ga), C.byref(da),
+                          self._ca_p, None, self._ctas, st), "dispatch+GEMM+combine launch")
+            if ev:
+                ev("dispatch+gemm+combine")
+
+        # 5. slot reduce + retire
+        y = torch.empty((T, cfg.out_dim), dtype=cfg.dtype, device=x.device)
+        n_tiles = (cfg.out_dim + BN - 1) // BN
+        nv.check(self._slot_reduce(self._out_slots_p, self._dst_slot_p, self._arrived_p, n * n_tiles, T, k, cfg.out_dim,
+                                   y.data_ptr(), self._ra_p, self._status_p, self._budget_ns, st), "slot reduce launch")
+        if ev:
+            ev("slot_reduce")
+        self._iteration += 1
+        self.last_routing = (idx, wgt)
+        return y
+
+    def _prepare_launches(self) -> None:
+        """Fill the argument blocks of a forward once per set of buffers: everything in them names buffers this
+        layer holds, so a forward only adds its own tensors (building them per call took 30 us of host time)."""
+        cfg, heap = self.cfg, self.heap
+        W, EL, ET, k, D = cfg.world_size, cfg.e_local, cfg.num_experts, cfg.topk, cfg.hidden_dim
+        iter_p, status_p = self.iter_dev.data_ptr(), heap.status.data_ptr()
+        esz = 2   # bytes per bf16
+        plan = self._plan
         push = PlanPushArgs()
         push.world, push.rank = W, heap.rank
         push.iter_done = self.iter_done.data_ptr()
@@ -447,41 +530,14 @@ class MoELayer(nn.Module):
         push.stride_flags = W * 4
         push.status = status_p
         push.wait_budget_ns = self._budget_ns
-        plan = self._plan
-        n = T * k
-        view = Plan(plan.counts, plan.bucket_start, plan.send_order[:n], plan.dst_slot[:n],
-                    plan.rank_in_bucket[:n])
-        if self.uses_small_path(T):
-            # 1+2. small batch: router and plan in one launch
-            idx = torch.empty((T, k), dtype=torch.int32, device=x.device)
-            wgt = torch.empty((T, k), dtype=torch.float32, device=x.device)
-            bias = None if self.router_bias is None else self.router_bias.to(
-                device=x.device, dtype=torch.float32).contiguous()
-            nv.check(self._route_plan_small(ptr(x), ptr(router_kmajor(self.router)), ptr(bias), T, D, ET, k,
-                                            int(cfg.renormalize), ptr(idx), ptr(wgt), ptr(view.counts),
-                                            ptr(view.bucket_start), ptr(view.send_order), ptr(view.dst_slot),
-                                            C.byref(push), ptr(self._small_ticket), st), "route+plan launch")
-            ev("router")
-            ev("plan")
-        else:
-            # 1. router
-            idx, wgt = self.route(x)
-            ev("router")
-            # 2. plan (+ counts push)
-            make_plan(idx, ET, out=view, push=push, workspace=self._plan_ws)
-            ev("plan")
 
-        # 3. dispatch + GEMM1 (one kernel)
         da = nv.DispatchArgs()
-        da.world, da.rank, da.e_local, da.topk, da.num_tokens = W, heap.rank, EL, k, T
-        da.x = x.data_ptr()
+        da.world, da.rank, da.e_local = W, heap.rank, EL
         da.send_order = plan.send_order.data_ptr()
-        da.topk_weight = wgt.data_ptr()
         da.counts_all = self.counts_all[0].data_ptr()
         da.counts_flag = self.counts_flag[0].data_ptr()
         da.cap_rows = self.cap_rows
         da.cap_mtiles = self.cap_mtiles
-        da.drop_signal = int(self.drop_signal)
         da.peer_recv = heap.peer_ptrs(self.recv[0])
         da.peer_meta = heap.peer_ptrs(self.meta[0])
         da.peer_ready = heap.peer_ptrs(self.ready[0])
@@ -492,12 +548,6 @@ class MoELayer(nn.Module):
         da.stride_meta = self.cap_rows * 8
         da.stride_ready = self.cap_mtiles * 4
         da.group_rows_out = self.group_rows.data_ptr()
-        if self.trace_arrivals:
-            if self._trace is None:
-                self._trace = torch.zeros(2 + 2 * self.cap_mtiles, dtype=torch.int64, device=x.device)
-            self._trace.zero_()
-            da.trace = self._trace.data_ptr()
-            da.trace_tiles = self.cap_mtiles
 
         ca = nv.CombineArgs()
         ca.world = W
@@ -510,45 +560,22 @@ class MoELayer(nn.Module):
         ca.peer_arrived = heap.peer_ptrs(self.arrived)
 
         ga = nv.GemmArgs()
-        ga.num_groups, ga.K, ga.group_m = EL, D, self.group_m[0]
+        ga.num_groups, ga.K = EL, D
         ga.status, ga.wait_budget_ns = status_p, self._budget_ns
         ga.cta_pair = self._cta_pair
-        # a prefetch ahead of the routing pays when every expert will be read
-        prefetch = 16 if T * k >= 4 * ET else 0
-        ga.l2_hints = self.l2_hints[0] | prefetch
-        ga.tma_store = 0 if self.tma_store else -1
-        ga.wide_tiles = self.wide_tiles[0]
-        recv = self.recv[0]
+        gb = None
         if cfg.gated:
             F = cfg.ffn_dim
             ga.N, ga.n_out = 2 * F, F
             ga.out, ga.ldo = self.hidden.data_ptr(), F
-            nv.check(lib.b200_grouped_gemm(ptr(recv), self.cap_rows, ptr(self.w13), nv.EPI_SILU_GATE, 1,
-                                           C.byref(ga), C.byref(da), None, None, self._ctas, st),
-                     "dispatch+GEMM1 launch")
-            ev("dispatch+gemm1")
-            # 4. GEMM2 + combine (one kernel)
             gb = nv.GemmArgs()
-            gb.num_groups, gb.N, gb.K, gb.n_out, gb.group_m = EL, D, F, D, self.group_m[1]
+            gb.num_groups, gb.N, gb.K, gb.n_out = EL, D, F, D
             gb.group_rows = self.group_rows.data_ptr()
             gb.status, gb.wait_budget_ns = status_p, self._budget_ns
             gb.cta_pair = self._cta_pair
-            gb.l2_hints = self.l2_hints[1] | prefetch
-            gb.wide_tiles = self.wide_tiles[1]
-            nv.check(lib.b200_grouped_gemm(ptr(self.hidden), self.cap_rows, ptr(self.w2), nv.EPI_COMBINE,
-                                           0, C.byref(gb), None, C.byref(ca), None, self._ctas, st),
-                     "GEMM2+combine launch")
-            ev("gemm2+combine")
         else:
-            # single Linear: dispatch, GEMM and combine are ONE kernel
             ga.N = ga.n_out = cfg.out_dim
-            nv.check(lib.b200_grouped_gemm(ptr(recv), self.cap_rows, ptr(self.w13), nv.EPI_COMBINE, 1,
-                                           C.byref(ga), C.byref(da), C.byref(ca), None, self._ctas, st),
-                     "dispatch+GEMM+combine launch")
-            ev("dispatch+gemm+combine")
 
-        # 5. slot reduce + retire
-        y = torch.empty((T, cfg.out_dim), dtype=cfg.dtype, device=x.device)
         ra = RetireArgs()
         ra.world, ra.rank = W, heap.rank
         ra.peer_iter_done = heap.peer_ptrs(self.iter_done)
@@ -557,15 +584,13 @@ class MoELayer(nn.Module):
         ra.stride_ready = self.cap_mtiles * 4
         ra.num_ready = self.cap_mtiles
         ra.ticket = self.ticket.data_ptr()
-        n_tiles = (cfg.out_dim + BN - 1) // BN
-        nv.check(self._slot_reduce(ptr(self.out_slots), ptr(plan.dst_slot), ptr(self.arrived),
-                                   T * k * n_tiles, T, k,
-                                   cfg.out_dim, ptr(y), C.byref(ra), C.c_void_p(status_p),
-                                   self._budget_ns, st), "slot reduce launch")
-        ev("slot_reduce")
-        self._iteration += 1
-        self.last_routing = (idx, wgt)
-        return y
+
+        self._gemm = nv.lib().b200_grouped_gemm
+        self._push, self._da, self._ca, self._ga, self._gb, self._ra = push, da, ca, ga, gb, ra
+        self._push_p, self._ca_p, self._ra_p = C.pointer(push), C.pointer(ca), C.pointer(ra)
+        self._plan_ptrs = tuple(t.data_ptr() for t in (plan.counts, plan.bucket_start, plan.send_order, plan.dst_slot))
+        self._recv_p, self._out_slots_p = self.recv.data_ptr(), self.out_slots.data_ptr()
+        self._dst_slot_p, self._arrived_p, self._status_p = plan.dst_slot.data_ptr(), self.arrived.data_ptr(), status_p
 
     # ------------------------------------------------------------ CUDA graphs
     def capture(self, num_tokens: Optional[int] = None) -> None:

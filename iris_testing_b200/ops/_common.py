@@ -14,8 +14,15 @@ def use_native(t: torch.Tensor) -> bool:
     return t.is_cuda
 
 
+# The raw handle of a device's current stream without building a Stream object, where torch has it.
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+
 def stream_ptr(t: torch.Tensor) -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    idx = t.get_device()
+    if _raw_stream is None or idx < 0:
+        return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    return C.c_void_p(_raw_stream(idx))
 
 
 def ptr(t) -> C.c_void_p:

@@ -74,6 +74,15 @@ class PaddedAllToAll:
         per_sm = 4 if self._plain else 1
         self.blocks = int(num_blocks) if num_blocks else sm_count(heap.device) * per_sm
         self.budget_ns = int(wait_budget_ms * 1e6)
+        # where every rank keeps the buffers above: fixed for their lifetime
+        b = self.buffers
+        self._peers = tuple(heap.peer_ptrs(t) for t in (b.pca, b.token_buf, b.counts_ready, b.token_sync, self.entered))
+        self._ret_peers = None if self.ret is None else (heap.peer_ptrs(self.ret.ret_buf), heap.peer_ptrs(self.ret.ret_sync))
+        self._exchange = _exchange_fn()
+        self._wait = declare("b200_padded_wait", [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,
+                                                  C.c_int, C.c_void_p, C.c_ulonglong, C.c_void_p])
+        self._pca_p, self._counts_p, self._sync_p, self._entered_p, self._status_p = (
+            t.data_ptr() for t in (b.pca, b.counts_ready, b.token_sync, self.entered, heap.status))
         torch.cuda.synchronize(heap.device)
         if W > 1:
             dist.barrier(group=heap.group)        # every rank's flags exist and are zero
@@ -96,37 +105,31 @@ class PaddedAllToAll:
                 "send_counts and dst_offsets must be int32")
         require(payload.is_contiguous() and payload.dtype == self.dtype and payload.shape[-1] == self.H,
                 "payload must be contiguous [rows, hidden_dim] of the buffer dtype")
-        h, b = self.heap, self.buffers
+        b = self.buffers
         self.epoch += 1
-        rc = _exchange_fn()(ptr(payload), ptr(send_counts), ptr(dst_offsets), h.peer_ptrs(b.pca),
-                            h.peer_ptrs(b.token_buf), h.peer_ptrs(b.counts_ready), h.peer_ptrs(b.token_sync),
-                            h.peer_ptrs(self.entered), ptr(self.entered), self.epoch, self.rank, self.world,
-                            self.e_local, self.cap, self.H, self.esz, tile_rows(), 0, self.blocks, self._plain,
-                            ptr(h.status), self.budget_ns, stream_ptr(payload))
+        rc = self._exchange(payload.data_ptr(), send_counts.data_ptr(), dst_offsets.data_ptr(), *self._peers,
+                            self._entered_p, self.epoch, self.rank, self.world, self.e_local, self.cap, self.H, self.esz,
+                            tile_rows(), 0, self.blocks, self._plain, self._status_p, self.budget_ns, stream_ptr(payload))
         nv.check(rc, "padded dispatch launch")
         return b.token_buf
 
     def wait(self) -> None:
         """Device-side wait (bounded) until this rank has received everything of the current
         dispatch; later work on the stream may read ``token_buf`` and ``pca``."""
-        b = self.buffers
-        fn = declare("b200_padded_wait", [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int,
-                                          C.c_int, C.c_void_p, C.c_ulonglong, C.c_void_p])
-        nv.check(fn(ptr(b.pca), ptr(b.counts_ready), ptr(b.token_sync), self.world, self.e_local, self.cap,
-                    tile_rows(), ptr(self.heap.status), self.budget_ns, stream_ptr(b.pca)), "padded wait launch")
+        nv.check(self._wait(self._pca_p, self._counts_p, self._sync_p, self.world, self.e_local, self.cap, tile_rows(),
+                            self._status_p, self.budget_ns, stream_ptr(self.buffers.pca)), "padded wait launch")
 
     def send_back(self, out_buf: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Return the processed rows ``out_buf[e_local, world(src), CAP, H]`` (default: the received
         ``token_buf`` itself) to their source ranks.  Call after :meth:`wait` (the counts must
         have landed).  Returns ``ret_buf`` without waiting for remote arrival."""
         require(self.ret is not None, "constructed without with_return=True")
-        h, b, r = self.heap, self.buffers, self.ret
+        b, r = self.buffers, self.ret
         src = b.token_buf if out_buf is None else out_buf
         require(src.is_contiguous() and tuple(src.shape) == tuple(b.token_buf.shape), "out_buf has the wrong shape")
-        rc = _exchange_fn()(ptr(src), ptr(b.pca), None, None, h.peer_ptrs(r.ret_buf), None,
-                            h.peer_ptrs(r.ret_sync), None, None, self.epoch, self.rank, self.world,
-                            self.e_local, self.cap, self.H, self.esz, tile_rows(), 1, self.blocks, self._plain,
-                            ptr(h.status), self.budget_ns, stream_ptr(src))
+        rc = self._exchange(src.data_ptr(), self._pca_p, None, None, self._ret_peers[0], None, self._ret_peers[1], None,
+                            None, self.epoch, self.rank, self.world, self.e_local, self.cap, self.H, self.esz, tile_rows(),
+                            1, self.blocks, self._plain, self._status_p, self.budget_ns, stream_ptr(src))
         nv.check(rc, "padded return launch")
         return r.ret_buf
 
