@@ -157,11 +157,14 @@ struct PaddedArgs {
   long long row_bytes;
   int mirror;
   int plain;       // 1: rows move as 16-byte loads/stores of all threads of a block instead of bulk copies
+  int split;       // plain: blocks that share a tile
+  uint32_t* parts; // plain: [2][parts_stride] shares of each tile that are done (epoch parity; local, zero at first)
+  int parts_stride;
   int* status;
   unsigned long long budget_ns;
 };
 
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 4)
 padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__ counts,
                    const int* __restrict__ dst_offsets, PaddedArgs a) {
   extern __shared__ __align__(128) uint8_t a2a_smem[];
@@ -171,6 +174,8 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int W = a.world, EL = a.e_local;
   if (tid == 0) s_abort = 0;
+  chain_wait();
+  if (!a.mirror) chain_release();    // next comes the one-block wait; behind a return a grid of many blocks
   if (lane == 0 && warp < A2A_WARPS) {
     mbar_init(&bars[warp][0], 1);
     mbar_init(&bars[warp][1], 1);
@@ -219,14 +224,20 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
   const int tpc = (a.cap + a.block_m - 1) / a.block_m;
   const long long total = static_cast<long long>(W) * EL * tpc;
   if (a.plain) {
-    // ---- tiles: one block per unit, every warp copies rows with eight 16-byte accesses in
-    // flight per lane; several blocks per SM hide each other's end-of-tile fence
+    // ---- tiles: one block per share of a tile, eight 16-byte accesses in flight per lane; several blocks per SM
+    // hide each other's end-of-share fence.  A tile is one contiguous block on both sides, so it is cut by
+    // bytes; a short message has fewer tiles than the chip has SMs (512 tokens of 4096: 36 tiles, 15 us whole,
+    // 7 us in eighths) and a long one an uneven number per SM.  The block that finishes a tile's last share
+    // counts the tile.
+    uint32_t* parts = a.parts + static_cast<size_t>(a.epoch & 1u) * a.parts_stride;
+    uint32_t* next = a.parts + static_cast<size_t>(~a.epoch & 1u) * a.parts_stride;
+    for (int i = blockIdx.x * blockDim.x + tid; i < a.parts_stride; i += gridDim.x * blockDim.x) next[i] = 0u;
     __shared__ unsigned s_entered;
     if (tid == 0) s_entered = a.mirror ? 0xffffffffu : 0u;
     __syncthreads();
-    const int nwarps = blockDim.x >> 5;
-    const int row16 = static_cast<int>(a.row_bytes / 16);
-    for (long long u = blockIdx.x; u < total; u += gridDim.x) {
+    for (long long v = blockIdx.x; v < total * a.split; v += gridDim.x) {
+      const long long u = v / a.split;
+      const int share = static_cast<int>(v - u * a.split);
       const int d = static_cast<int>(u % W);
       const long long rest = u / W;
       const int e = static_cast<int>(rest % EL), mt = static_cast<int>(rest / EL);
@@ -237,7 +248,10 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
       const int m0 = mt * a.block_m;
       if (m0 >= n) continue;
       const int rows = min(a.block_m, n - m0);
-      if (!(s_entered >> peer & 1u)) {          // uniform: s_entered only changes between barriers
+      // A peer's buffers may be written once it has entered the epoch.  This rank's own rows may go at once (their
+      // consumer ran earlier in this stream); only the count has to come after the flags were re-armed.
+      const bool need = !(s_entered >> peer & 1u);   // uniform for peers: their bits change between barriers
+      if (need && peer != a.rank) {
         if (tid == 0 && wait_flag_geq(a.entered_local + peer, a.epoch, w, ST_TIMEOUT_BARRIER))
           s_entered |= 1u << peer;
         __syncthreads();
@@ -254,13 +268,39 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
         dst = reinterpret_cast<uint8_t*>(a.token_buf.p[peer]) +
               ((static_cast<long long>(a.rank) * EL + e) * a.cap + m0) * a.row_bytes;
       }
-      for (int r = warp; r < rows; r += nwarps)
-        copy_row_16(reinterpret_cast<uint4*>(dst + r * a.row_bytes),
-                    reinterpret_cast<const uint4*>(src + r * a.row_bytes), row16, lane);
+      const long long pieces = rows * a.row_bytes / 16, per = (pieces + a.split - 1) / a.split;
+      const long long hi = min(pieces, (share + 1) * per);
+      const uint4* s4 = reinterpret_cast<const uint4*>(src);
+      uint4* d4 = reinterpret_cast<uint4*>(dst);
+      for (long long i = share * per + tid; i < hi; i += 8 * blockDim.x) {
+        uint4 x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (i + j * static_cast<int>(blockDim.x) < hi) x[j] = ld_16(s4 + i + j * static_cast<int>(blockDim.x));
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (i + j * static_cast<int>(blockDim.x) < hi) st_16(d4 + i + j * static_cast<int>(blockDim.x), x[j]);
+      }
       __syncthreads();
       if (tid == 0) {
-        fence_acq_rel_sys();
-        red_add_release_sys(reinterpret_cast<uint32_t*>(a.token_sync.p[peer]) + (a.mirror ? a.rank : e), 1u);
+        bool ok = true;
+        if (need && peer == a.rank) {
+          ok = wait_flag_geq(a.entered_local + peer, a.epoch, w, ST_TIMEOUT_BARRIER);
+          if (ok) s_entered |= 1u << peer;
+        }
+        if (ok) {
+          if (peer == a.rank) fence_acq_rel_gpu(); else fence_acq_rel_sys();
+          bool last = true;
+          if (a.split > 1) {
+            last = atomicAdd(parts + u, 1u) + 1u == static_cast<unsigned>(a.split);
+            if (last) {
+              parts[u] = 0u;       // (an epoch that was given up leaves its counters to the next epoch's clearing)
+              if (peer == a.rank) fence_acq_rel_gpu(); else fence_acq_rel_sys();
+            }
+          }
+          uint32_t* flag = reinterpret_cast<uint32_t*>(a.token_sync.p[peer]) + (a.mirror ? a.rank : e);
+          if (last) { if (peer == a.rank) red_add_relaxed_gpu(flag, 1u); else red_add_relaxed_sys(flag, 1u); }
+        }
       }
     }
     return;
@@ -346,6 +386,8 @@ __global__ void padded_wait_kernel(const int* pca, const uint32_t* counts_ready,
                                    unsigned long long budget_ns) {
   __shared__ int s_abort;
   if (threadIdx.x == 0) s_abort = 0;
+  chain_wait();
+  chain_release();
   __syncthreads();
   WaitCtx w; w.abort_flag = &s_abort; w.status = status; w.budget_ns = budget_ns;
   if (threadIdx.x == 0) wait_flag_geq(counts_ready, static_cast<uint32_t>(world), w, ST_TIMEOUT_COUNTS);
@@ -379,6 +421,7 @@ weighted_gather_kernel(const __nv_bfloat16* __restrict__ ret_buf,
   __shared__ int s_abort;
   __shared__ int s_last;
   if (threadIdx.x == 0) s_abort = 0;
+  chain_wait();
   __syncthreads();
   if (threadIdx.x < world) {
     uint32_t expect = 0;
@@ -763,6 +806,8 @@ int b200_padded_return(const void* out_buf, const int* pca, const unsigned long 
 // dispatch: rows = packed payload, counts = send_counts [world, e_local], dst_offsets [world];
 // return:   rows = out_buf [e_local, world, cap, H], counts = pca [e_local, world], dst_offsets unused,
 //           peer_token_buf = ret_buf, peer_token_sync = ret_sync.
+// parts: [2][parts_stride] zeroed words of this rank's memory for this direction, one per tile; split: blocks per tile
+// (plain copies; 1 without parts).
 int b200_padded_exchange(const void* rows, const int* counts, const int* dst_offsets,
                          const unsigned long long* peer_pca, const unsigned long long* peer_token_buf,
                          const unsigned long long* peer_counts_ready,
@@ -770,7 +815,7 @@ int b200_padded_exchange(const void* rows, const int* counts, const int* dst_off
                          const unsigned long long* peer_entered, const void* entered_local,
                          unsigned int epoch, int rank, int world, int e_local, int cap, int hidden_dim,
                          int elem_bytes, int block_m, int mirror, int num_blocks, int plain, int* status,
-                         unsigned long long budget_ns, void* stream) {
+                         unsigned long long budget_ns, void* parts, int parts_stride, int split, void* stream) {
   if (world < 1 || world > B200_MAX_WORLD || world * e_local > B200_MAX_EXPERTS || block_m < 1 || cap < 1 ||
       (static_cast<long long>(hidden_dim) * elem_bytes) % 16 != 0 || num_blocks < 1 ||
       (reinterpret_cast<uintptr_t>(rows) & 15u) != 0)
@@ -797,27 +842,31 @@ int b200_padded_exchange(const void* rows, const int* counts, const int* dst_off
   a.row_bytes = static_cast<long long>(hidden_dim) * elem_bytes;
   a.mirror = mirror;
   a.plain = plain ? 1 : 0;
+  a.parts = static_cast<uint32_t*>(parts);
+  a.parts_stride = parts != nullptr ? parts_stride : 0;
+  // a tile is only shared where its counter exists (the caller sized them for some block_m)
+  const long long tiles = static_cast<long long>(world) * e_local * ((cap + block_m - 1) / block_m);
+  a.split = split > 1 && tiles <= a.parts_stride ? split : 1;
   a.status = status;
   a.budget_ns = budget_ns;
-  if (plain)
-    b200::padded_bulk_kernel<<<num_blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(rows), counts, dst_offsets, a);
-  else
-    b200::padded_bulk_kernel<<<num_blocks, b200::A2A_WARPS * 32, smem, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const uint8_t*>(rows), counts, dst_offsets, a);
+  const cudaError_t e = b200::launch_chained(b200::padded_bulk_kernel, dim3(num_blocks),
+                                             dim3(plain ? 256 : b200::A2A_WARPS * 32), plain ? 0 : smem,
+                                             static_cast<cudaStream_t>(stream), static_cast<const uint8_t*>(rows), counts,
+                                             dst_offsets, a);
   b200_count_launches(1);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(e);
 }
 
 int b200_padded_wait(const int* pca, const void* counts_ready, const void* token_sync, int world,
                      int e_local, int cap, int block_m, int* status, unsigned long long budget_ns,
                      void* stream) {
   if (world < 1 || e_local < 1 || block_m < 1) return -1;
-  b200::padded_wait_kernel<<<1, 128, 0, static_cast<cudaStream_t>(stream)>>>(
-      pca, static_cast<const uint32_t*>(counts_ready), static_cast<const uint32_t*>(token_sync), world,
-      e_local, cap, block_m, status, budget_ns);
+  const cudaError_t e = b200::launch_chained(
+      b200::padded_wait_kernel, dim3(1), dim3(128), 0, static_cast<cudaStream_t>(stream), pca,
+      static_cast<const uint32_t*>(counts_ready), static_cast<const uint32_t*>(token_sync), world, e_local, cap, block_m,
+      status, budget_ns);
   b200_count_launches(1);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(e);
 }
 
 int b200_weighted_gather(const void* ret_buf, const int* dst_slot, const int* topk_idx,
@@ -829,11 +878,12 @@ int b200_weighted_gather(const void* ret_buf, const int* dst_slot, const int* to
   int blocks = (T + 7) / 8;
   if (blocks < 1) blocks = 1;
   if (blocks > 148 * 8) blocks = 148 * 8;
+  cudaError_t err = cudaSuccess;
   auto go = [&](auto kern) {
-    kern<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(ret_buf), dst_slot, topk_idx, bucket_start, topk_w,
-        static_cast<uint32_t*>(ret_sync), send_counts, T, topk, world, e_local, cap, hidden_dim,
-        block_m, static_cast<__nv_bfloat16*>(y), status, budget_ns, ticket);
+    err = b200::launch_chained(kern, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                               static_cast<const __nv_bfloat16*>(ret_buf), dst_slot, topk_idx, bucket_start, topk_w,
+                               static_cast<uint32_t*>(ret_sync), send_counts, T, topk, world, e_local, cap, hidden_dim,
+                               block_m, static_cast<__nv_bfloat16*>(y), status, budget_ns, ticket);
   };
   const bool wide = hidden_dim > 1024;
   if (topk == 1) wide ? go(b200::weighted_gather_kernel<1, 4>) : go(b200::weighted_gather_kernel<1, 1>);
@@ -841,7 +891,7 @@ int b200_weighted_gather(const void* ret_buf, const int* dst_slot, const int* to
   else if (topk <= 4) wide ? go(b200::weighted_gather_kernel<4, 2>) : go(b200::weighted_gather_kernel<4, 1>);
   else go(b200::weighted_gather_kernel<8, 1>);
   b200_count_launches(1);
-  return static_cast<int>(cudaGetLastError());
+  return static_cast<int>(err);
 }
 
 int b200_shuffle(void* token_buf, void* packed, const int* pca, const void* counts_ready,

@@ -35,7 +35,7 @@ def _exchange_fn():
     return declare("b200_padded_exchange",
                    [C.c_void_p, C.c_void_p, C.c_void_p, u64p, u64p, u64p, u64p, u64p, C.c_void_p, C.c_uint,
                     C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
-                    C.c_void_p, C.c_ulonglong, C.c_void_p])
+                    C.c_void_p, C.c_ulonglong, C.c_void_p, C.c_int, C.c_int, C.c_void_p])
 
 
 class PaddedAllToAll:
@@ -74,6 +74,11 @@ class PaddedAllToAll:
         per_sm = 4 if self._plain else 1
         self.blocks = int(num_blocks) if num_blocks else sm_count(heap.device) * per_sm
         self.budget_ns = int(wait_budget_ms * 1e6)
+        # "stores": progress of tiles that several blocks share, per direction (csrc/exchange.cu padded_bulk_kernel)
+        self._tiles = W * self.e_local * (-(-self.cap // tile_rows()))
+        self._parts = torch.zeros((2, 2, self._tiles), dtype=i32, device=heap.device)
+        self._parts_p = (self._parts[0].data_ptr(), self._parts[1].data_ptr())
+        self._split = 1
         # where every rank keeps the buffers above: fixed for their lifetime
         b = self.buffers
         self._peers = tuple(heap.peer_ptrs(t) for t in (b.pca, b.token_buf, b.counts_ready, b.token_sync, self.entered))
@@ -107,9 +112,15 @@ class PaddedAllToAll:
                 "payload must be contiguous [rows, hidden_dim] of the buffer dtype")
         b = self.buffers
         self.epoch += 1
+        bm = tile_rows()
+        # blocks per tile: up to eight, until there are as many shares as blocks
+        tiles, self._split = max(payload.shape[0] // bm, 1), 1
+        while self._split < 8 and tiles * self._split < self.blocks:
+            self._split *= 2
         rc = self._exchange(payload.data_ptr(), send_counts.data_ptr(), dst_offsets.data_ptr(), *self._peers,
                             self._entered_p, self.epoch, self.rank, self.world, self.e_local, self.cap, self.H, self.esz,
-                            tile_rows(), 0, self.blocks, self._plain, self._status_p, self.budget_ns, stream_ptr(payload))
+                            bm, 0, self.blocks, self._plain, self._status_p, self.budget_ns, self._parts_p[0], self._tiles,
+                            self._split, stream_ptr(payload))
         nv.check(rc, "padded dispatch launch")
         return b.token_buf
 
@@ -129,7 +140,8 @@ class PaddedAllToAll:
         require(src.is_contiguous() and tuple(src.shape) == tuple(b.token_buf.shape), "out_buf has the wrong shape")
         rc = self._exchange(src.data_ptr(), self._pca_p, None, None, self._ret_peers[0], None, self._ret_peers[1], None,
                             None, self.epoch, self.rank, self.world, self.e_local, self.cap, self.H, self.esz, tile_rows(),
-                            1, self.blocks, self._plain, self._status_p, self.budget_ns, stream_ptr(src))
+                            1, self.blocks, self._plain, self._status_p, self.budget_ns, self._parts_p[1], self._tiles,
+                            self._split, stream_ptr(src))
         nv.check(rc, "padded return launch")
         return r.ret_buf
 

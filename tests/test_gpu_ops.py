@@ -360,3 +360,36 @@ def test_weighted_gather_row_groups(dev, T, k, E, H, drop):
     ref = (rows * (w.reshape(-1, 1).double() * (m < cap).unsqueeze(1))).view(T, k, H).sum(1)
     mag = (rows.abs() * w.reshape(-1, 1).double()).view(T, k, H).sum(1)
     assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + mag * k * 2.0 ** -23).all())
+
+
+@pytest.mark.parametrize("T,k,H", [(1, 1, 8), (33, 2, 136), (300, 2, 4096), (2400, 2, 264), (4800, 2, 72), (9500, 2, 64)])
+def test_padded_exchange_shares_of_tiles(dev, T, k, H):
+    """Tiles shared by eight, four and two blocks and by none, another share count from call to call, a
+    dispatch whose return is left out: rows bit-equal, every tile counted once."""
+    from iris_testing_b200.parallel.padded_a2a import PaddedAllToAll
+    from iris_testing_b200.parallel.symm import SymmetricHeap
+    from iris_testing_b200.utils import gen_local_tokens, gen_router, route_and_pack
+    E = 4
+    heap = SymmetricHeap(2 * E * T * H * 2 + (32 << 20))
+    a2a = PaddedAllToAll(heap, E, T, H, torch.bfloat16, with_return=True)
+    router = gen_router(H, E, torch.bfloat16, dev, 3, std=None)
+    for i, n in enumerate((T, max(T // 9, 1), T, T)):
+        x = gen_local_tokens(1, n, H, torch.bfloat16, dev, i, 0, "normal")
+        payload, counts, dst_off, _, idx, wgt, plan = route_and_pack(x, router, k, 1, E)
+        out = a2a.dispatch(payload, counts, dst_off)
+        a2a.wait()
+        assert torch.equal(a2a.token_sync, ((counts.reshape(-1) + 31) // 32).to(torch.int32))
+        cells = torch.cat([out[e, 0, :c] for e, c in enumerate(counts.reshape(-1).tolist())])
+        assert torch.equal(cells, payload)
+        if i != 1:
+            a2a.send_back()
+            y = a2a.reduce(plan, idx, wgt)
+            back = torch.cat([a2a.ret.ret_buf[0, e, :c] for e, c in enumerate(counts.reshape(-1).tolist())])
+            assert torch.equal(back, payload) and int(a2a.ret.ret_sync.abs().sum()) == 0
+            ref = x.double() * wgt.double().sum(1, keepdim=True)
+            mag = x.double().abs() * wgt.double().sum(1, keepdim=True)     # bf16 rounding, fp32 sums of k products
+            assert bool(((y.double() - ref).abs() <= mag * (2.0 ** -8 + k * 2.0 ** -22)).all())
+        assert int(a2a._parts.abs().sum()) == 0
+    heap.check_status()
+    del a2a
+    heap.close()
