@@ -590,7 +590,8 @@ struct RetireArgs {
 // a token's row is split over `wpt` warps while SMs are idle, and whatever does not depend on the arrivals (row
 // numbers, iteration, status) is read before or along with the first look at their counter.
 template <int KMAX>   // topk <= KMAX; about eight 16-byte loads per lane are kept in flight
-__global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __restrict__ dst_slot,
+__global__ void __launch_bounds__(256, 4)
+slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __restrict__ dst_slot,
                                    uint32_t* arrived, uint32_t expected, int T, int topk, int H,
                                    __nv_bfloat16* __restrict__ y, RetireArgs ra, int* status,
                                    unsigned long long budget_ns, int wpt) {
@@ -601,15 +602,13 @@ __global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __
   const int part = warp % wpt;     // this warp's share of a token's columns
   chain_wait();
   // results sit at the row's position in the packed send order (dst_slot), or at t*topk+s when no map is given
-  size_t row[KMAX];
+  int row[KMAX], next[KMAX];
   auto find_rows = [&](int t) {
 #pragma unroll
     for (int s = 0; s < KMAX; ++s)
-      if (s < topk)
-        row[s] = dst_slot != nullptr ? static_cast<size_t>(__ldg(dst_slot + t * topk + s))
-                                     : static_cast<size_t>(t) * topk + s;
+      if (s < topk && t < T) next[s] = dst_slot != nullptr ? __ldg(dst_slot + t * topk + s) : t * topk + s;
   };
-  if (warp / wpt < T) find_rows(warp / wpt);
+  find_rows(warp / wpt);
   if (threadIdx.x == 32) s_iter = ra.iter_ptr != nullptr ? __ldcg(ra.iter_ptr) : 0u;
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -627,10 +626,10 @@ __global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __
   __syncthreads();
   if (!s_abort) {
     constexpr int U = 8 / KMAX;    // 16-byte column chunks per lane in flight at once (times topk loads)
-    bool first = true;
     for (int t = warp / wpt; t < T; t += nwarps / wpt) {
-      if (!first) find_rows(t);
-      first = false;
+#pragma unroll
+      for (int s = 0; s < KMAX; ++s) row[s] = next[s];
+      find_rows(t + nwarps / wpt);          // the next token's row numbers travel behind this one's rows
       for (int cb = part * 256 * U + lane * 8; cb < H; cb += 256 * U * wpt) {
         uint4 v[U][KMAX];
 #pragma unroll
@@ -639,7 +638,7 @@ __global__ void slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __
 #pragma unroll
           for (int s = 0; s < KMAX; ++s)
             if (s < topk && c0 < H)
-              v[u][s] = ld_16(reinterpret_cast<const uint4*>(out_slots + row[s] * H + c0));
+              v[u][s] = ld_16(reinterpret_cast<const uint4*>(out_slots + static_cast<size_t>(row[s]) * H + c0));
         }
 #pragma unroll
         for (int u = 0; u < U; ++u) {
