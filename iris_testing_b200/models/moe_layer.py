@@ -36,7 +36,7 @@ from .. import _native as nv
 from ..config import MoEConfig
 from ..ops import cpu_ref
 from ..ops._common import declare, ptr, stream_ptr
-from ..ops.expert import sm_count
+from ..ops.expert import pairs_pay, sm_count
 from ..ops.plan import Plan, PlanPushArgs, make_plan, plan_workspace
 from ..ops.router import router_kmajor, router_topk
 from ..utils import gen
@@ -227,12 +227,7 @@ class MoELayer(nn.Module):
         pair = cfg.cta_pair
         if os.getenv("B200MOE_CTA_PAIR", "") in ("0", "1"):       # override for tile-shape experiments
             pair = os.environ["B200MOE_CTA_PAIR"] == "1"
-        if pair is None:
-            # 256-row tiles pay off once experts average 128 rows: from there on many experts hold more than
-            # one 128-row tile, and a second tile streams the expert's weights again (Mixtral shape, one GPU:
-            # 700 -> 666 us at 128 rows per expert, 773 -> 670 us at 192; 555 -> 643 us at 64)
-            pair = (T * k * W) // max(ET, 1) >= 128
-        self._cta_pair = int(bool(pair))
+        self._cta_pair = pair                       # None: per call, by the rows per expert
         self._budget_ns = int(cfg.wait_budget_ms * 1e6)
         self.recv = self.meta = self.ready = self.hidden = None
         self._alloc_capacity(cap)
@@ -390,6 +385,14 @@ class MoELayer(nn.Module):
         the small-token path), fused GEMM kernel(s), slot reduce."""
         return (1 if self.uses_small_path(T) else 3) + (2 if self.cfg.gated else 1) + 1
 
+    def _uses_pairs(self, T: int) -> int:
+        """1 when the GEMM kernels of a forward of ``T`` tokens run on CTA pairs (256-row tiles)."""
+        cfg = self.cfg
+        if self._cta_pair is not None:
+            return int(bool(self._cta_pair))
+        rows = T * cfg.topk * cfg.world_size / cfg.num_experts
+        return int(rows >= 128 if any(self.wide_tiles) else pairs_pay(rows))
+
     @property
     def launches_per_forward(self) -> int:
         return self.launches_for(self.max_tokens)
@@ -479,6 +482,7 @@ class MoELayer(nn.Module):
         ga.l2_hints = self.l2_hints[0] | prefetch
         ga.tma_store = 0 if self.tma_store else -1
         ga.wide_tiles = self.wide_tiles[0]
+        ga.cta_pair = pair = self._uses_pairs(T)
         gemm = self._gemm
         if cfg.gated:
             nv.check(gemm(self._recv_p, self.cap_rows, self.w13.data_ptr(), nv.EPI_SILU_GATE, 1, C.byref(ga), C.byref(da),
@@ -490,6 +494,7 @@ class MoELayer(nn.Module):
             gb.group_m = self.group_m[1]
             gb.l2_hints = self.l2_hints[1] | prefetch
             gb.wide_tiles = self.wide_tiles[1]
+            gb.cta_pair = pair
             nv.check(gemm(self.hidden.data_ptr(), self.cap_rows, self.w2.data_ptr(), nv.EPI_COMBINE, 0, C.byref(gb), None,
                           self._ca_p, None, self._ctas, st), "GEMM2+combine launch")
             if ev:
@@ -562,7 +567,6 @@ class MoELayer(nn.Module):
         ga = nv.GemmArgs()
         ga.num_groups, ga.K = EL, D
         ga.status, ga.wait_budget_ns = status_p, self._budget_ns
-        ga.cta_pair = self._cta_pair
         gb = None
         if cfg.gated:
             F = cfg.ffn_dim
@@ -572,7 +576,6 @@ class MoELayer(nn.Module):
             gb.num_groups, gb.N, gb.K, gb.n_out = EL, D, F, D
             gb.group_rows = self.group_rows.data_ptr()
             gb.status, gb.wait_budget_ns = status_p, self._budget_ns
-            gb.cta_pair = self._cta_pair
         else:
             ga.N = ga.n_out = cfg.out_dim
 

@@ -27,6 +27,18 @@ def sm_count(device: torch.device) -> int:
     return _SM_COUNT[idx]
 
 
+def pairs_pay(rows: float) -> bool:
+    """Whether CTA pairs (256-row tiles) beat single CTAs (128-row tiles) at this average of rows per group.
+
+    From 128 rows on many groups hold more than one 128-row tile, and a second tile streams the
+    group's weights again (Mixtral shape on one B200, single / pair: 558 / 648 us at 100 rows per expert, 733 / 658 at
+    128, 821 / 672 at 160, 813 / 670 at 225).  Just above 256 rows most groups would fill a
+    second 256-row tile by less than half, and three 128-row tiles are less padding (1093 / 1164 us at
+    275 rows, 1131 / 1207 at 300, 1148 / 1275 at 350; 64 fine-grained experts 562 / 574 at 300); towards 384 that
+    is used up (589 / 589, one Linear 568 / 540) and from 512 on pairs win again (1575 / 1513)."""
+    return rows >= 128 and not 256 < rows <= 352
+
+
 def to_kmajor(weights: torch.Tensor) -> torch.Tensor:
     """[G, K, N] ("x @ W" layout, as the reference generates) -> [G, N, K] contiguous."""
     return weights.transpose(1, 2).contiguous()
@@ -58,7 +70,7 @@ def grouped_gemm(a: torch.Tensor, w_kmajor: torch.Tensor, group_rows: torch.Tens
     group_rows int32 [G] on the device (rows per group; sum <= M)
     group_m    M-tiles per L2-blocking chunk; 0 picks about 48 MB of activations per chunk.
     cta_pair   True: two CTAs per MMA (tcgen05 cta_group::2, 256-row tiles); None picks it
-               when the groups average at least 128 rows.
+               by the average rows per group (:func:`pairs_pay`).
     wide_tiles CTA pairs only: 512-column tiles that use both TMEM accumulators at once (25 % fewer
                operand bytes per FLOP, but the epilogue is no longer hidden); 1 = on, 0 = off (default).
     epilogue   EPI_STORE -> out [M, N];  EPI_SILU_GATE -> out [M, N/2] where every
@@ -104,7 +116,7 @@ def grouped_gemm(a: torch.Tensor, w_kmajor: torch.Tensor, group_rows: torch.Tens
     ga.status = status.data_ptr()
     ga.wait_budget_ns = int(wait_budget_ms * 1e6)
     if cta_pair is None:
-        cta_pair = M >= 128 * G
+        cta_pair = M >= 128 * G if wide_tiles else pairs_pay(M / G)
     ga.cta_pair = int(bool(cta_pair))
     ga.l2_hints = int(l2_hints)
     ga.wide_tiles = int(wide_tiles)

@@ -367,3 +367,16 @@ def test_slot_reduction_splits_rows_over_warps(D, k, T):
     for x, y in zip(xs, ys):
         _close(layer, x, y)
     _finish(layer)
+
+
+@pytest.mark.parametrize("rows", [127, 128, 256, 257, 352, 353])
+def test_tile_geometry_follows_the_rows_of_each_call(rows):
+    """Both sides of the lines between single CTAs and CTA pairs, in one layer made for more tokens."""
+    from iris_testing_b200.config import MoEConfig
+    from iris_testing_b200.utils import gen_local_tokens
+    cfg = MoEConfig(hidden_dim=128, ffn_dim=256, num_experts=4, topk=1)
+    layer, heap = _make(cfg, 3000)
+    assert layer._uses_pairs(4 * rows) == (128 <= rows and not 256 < rows <= 352)
+    x = gen_local_tokens(1, 4 * rows, 128, torch.bfloat16, heap.device, rows, 0, "normal")
+    _close(layer, x, layer(x))
+    _finish(layer)
