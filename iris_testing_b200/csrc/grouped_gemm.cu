@@ -10,7 +10,7 @@
 //   warp 0      TMA producer (one lane)
 //   warp 1      TMEM owner + MMA issuer (one lane)
 //   warps 2-5   epilogue: TMEM -> registers -> shared staging -> coalesced stores
-//   warps 6-9   (fused-dispatch build only) token senders: gather this rank's
+//   warps 6-13  (fused-dispatch build only) token senders: gather this rank's
 //               routed rows and store them into the owning rank's receive
 //               buffer over NVLink, then signal the M-tile they landed in.
 //
