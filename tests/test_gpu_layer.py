@@ -380,3 +380,41 @@ def test_tile_geometry_follows_the_rows_of_each_call(rows):
     x = gen_local_tokens(1, 4 * rows, 128, torch.bfloat16, heap.device, rows, 0, "normal")
     _close(layer, x, layer(x))
     _finish(layer)
+
+
+def test_capture_between_a_fork_and_a_join():
+    """Chained launches under capture: the layer's first kernel joins two branches, its last one is joined by a
+    third, and other kernels run before and after it on the same stream."""
+    from iris_testing_b200.config import MoEConfig
+    from iris_testing_b200.utils import gen_local_tokens
+    for T, gated in ((300, True), (300, False)):
+        cfg = MoEConfig(hidden_dim=256, ffn_dim=256 if gated else 0, num_experts=8, topk=2, gated=gated)
+        layer, heap = _make(cfg, T)
+        dev = heap.device
+        a = gen_local_tokens(1, T, 256, torch.bfloat16, dev, 5, 0, "normal")
+        b = torch.zeros_like(a)
+        layer((a + b))
+        torch.cuda.synchronize()
+        side = torch.cuda.Stream(dev)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            cur = torch.cuda.current_stream()
+            side.wait_stream(cur)
+            with torch.cuda.stream(side):
+                c = a * 1.0
+            d = b + 0.0
+            cur.wait_stream(side)
+            x = c + d
+            y = layer(x) + 0
+            side.wait_stream(cur)
+            with torch.cuda.stream(side):
+                z = y * 2.0
+            cur.wait_stream(side)
+        for i in range(3):
+            a.copy_(gen_local_tokens(1, T, 256, torch.bfloat16, dev, 40 + i, 0, "normal"))
+            g.replay()
+            torch.cuda.synchronize()
+            _close(layer, a, y)
+            assert torch.equal(z, y * 2.0)
+        _finish(layer)
+        del g
