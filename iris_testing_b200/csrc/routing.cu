@@ -97,19 +97,6 @@ __global__ void router_topk_simple_kernel(const __nv_bfloat16* __restrict__ x,
   }
 }
 
-// Router of every batch the small-token path does not take (see router_mma.cuh); one tile of tokens
-// per CTA.
-template <int NT, int KS>
-__global__ void __launch_bounds__(KS * 32, KS > 8 ? 1 : 2)
-router_mma_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wr_kmajor,
-                  const float* __restrict__ bias, int T, int D, int E, int k, int renorm,
-                  int* __restrict__ topk_idx, float* __restrict__ topk_w) {
-  extern __shared__ __align__(16) float router_smem[];
-  chain_wait();
-  chain_release();
-  route_tile<NT, KS>(x, wr_kmajor, bias, T, D, E, k, renorm, -1, blockIdx.x * 16, topk_idx, topk_w, router_smem);
-}
-
 // ---------------------------------------------------------------------------
 // Plan, step 1: one CTA per expert walks the flat (token, slot) list in order
 // and gives every copy routed to that expert its stable rank in the bucket.
@@ -574,38 +561,6 @@ int b200_router_topk_simple(const void* x, const void* wr, const float* bias, in
       renorm, topk_idx, topk_w, logits_out);
   b200_count_launches(1);
   return static_cast<int>(cudaGetLastError());
-}
-
-// Tensor-core router: wr_kmajor is the router matrix as [E, D].  Returns -2 when x or wr_kmajor is not
-// 16-byte aligned.
-int b200_router_mma(const void* x, const void* wr_kmajor, const b200_router_args* ra, int T, int D, void* stream) {
-  using namespace b200;
-  if (ra == nullptr || D < 8 || D % 8 != 0 || T < 0 || ra->num_experts < 1 || ra->num_experts > 256 || ra->topk < 1 ||
-      ra->topk > ROUTER_MAX_K || ra->topk > ra->num_experts)
-    return -1;
-  if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wr_kmajor)) & 15u) != 0) return -2;
-  if (T == 0) return 0;
-  const int E = ra->num_experts;
-  // A batch of up to 16 tokens per SM is one wave of CTAs: sixteen warps share a tile's rows and need
-  // half the dependent trips of eight.  Larger batches run two CTAs of eight warps per SM, except with
-  // more than 32 experts, where the expert rows through L1 are the limit and two CTAs gain nothing
-  // (4096 x 2048 tokens, 64 experts: 26 us with eight warps, 18 us with sixteen).
-  const bool big = T > 16 * 148;
-  auto go = [&](auto kern, int threads, int smem) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    e = launch_chained(kern, dim3((T + 15) / 16), dim3(threads), smem, static_cast<cudaStream_t>(stream),
-                       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(wr_kmajor), ra->bias, T,
-                       D, E, ra->topk, ra->renorm, ra->topk_idx, ra->topk_w);
-    b200_count_launches(1);
-    return static_cast<int>(e);
-  };
-#define B200_ROUTER(NT, KS) go(router_mma_kernel<NT, KS>, KS * 32, RouterTile<NT, KS>::smem_bytes(E))
-  if (E <= 8) return big ? B200_ROUTER(1, 8) : B200_ROUTER(1, 16);
-  if (E <= 16) return big ? B200_ROUTER(2, 8) : B200_ROUTER(2, 16);
-  if (E <= 32) return big ? B200_ROUTER(4, 8) : B200_ROUTER(4, 16);
-  return B200_ROUTER(8, 16);
-#undef B200_ROUTER
 }
 
 // Ints of workspace b200_plan_ws needs for lists of any length.

@@ -24,8 +24,8 @@ def router_topk(x: torch.Tensor, w_router: torch.Tensor, topk: int,
                 status: Optional[torch.Tensor] = None):
     """x [T, D], w_router [D, E] -> (idx int32 [T, k], weight fp32 [T, k][, logits fp32 [T, E]]).
 
-    On CUDA the logits are computed on the tensor cores and softmax/top-k run in the same
-    kernel (hidden_dim % 8 == 0 and E <= 256); other shapes, ``return_logits``
+    On CUDA the logits are computed on the tensor cores and softmax/top-k run in that
+    kernel's epilogue (hidden_dim % 8 == 0 and E <= 256); other shapes, ``return_logits``
     and ``force_simple`` take a CUDA-core kernel."""
     require(x.dim() == 2 and w_router.dim() == 2 and x.shape[1] == w_router.shape[0],
             "router_topk: x must be [T, D] and w_router [D, E]")
@@ -78,30 +78,12 @@ def router_kmajor(w_router: torch.Tensor) -> torch.Tensor:
     return t
 
 
-# 128-token tcgen05 tiles take over where the 16-token tiles' reads of the expert rows through L1 (once per
-# tile) become the limit: many experts and many tokens.  Measured with 2048-wide tokens, 16-token against
-# 128-token tiles: 64 experts 10 / 25 us at 2368 tokens, 57 / 27 us at 16384; 32 experts 30 / 21 us at
-# 16384; with 8 experts the 16-token tiles always win (16384 x 4096: 31 / 37 us).
-def _takes_tile128(tokens: int, experts: int) -> bool:
-    return experts > 16 and tokens * (2 if experts > 32 else 1) > 4 * 16 * 148
-
-
 def _router_tensor_core(x, wr_kmajor, bias, topk, renormalize, idx, w, status=None) -> None:
-    """Logits on the tensor cores, softmax and top-k in the same kernel (csrc/router_mma.cuh)."""
-    if _takes_tile128(x.shape[0], wr_kmajor.shape[0]):
-        return _router_tile128(x, wr_kmajor, bias, topk, renormalize, idx, w, status)
-    ra = nv.RouterArgs()
-    ra.num_experts, ra.topk, ra.renorm = wr_kmajor.shape[0], topk, int(renormalize)
-    ra.bias = None if bias is None else bias.data_ptr()
-    ra.topk_idx, ra.topk_w = idx.data_ptr(), w.data_ptr()
-    fn = declare("b200_router_mma", [C.c_void_p, C.c_void_p, C.POINTER(nv.RouterArgs), C.c_int, C.c_int, C.c_void_p])
-    nv.check(fn(ptr(x), ptr(wr_kmajor), C.byref(ra), x.shape[0], x.shape[1], stream_ptr(x)),
-             "tensor-core router launch")
-
-
-def _router_tile128(x, wr_kmajor, bias, topk, renormalize, idx, w, status=None) -> None:
     """Logits on tcgen05 (the grouped GEMM with one group and a narrow MMA), softmax and
-    top-k in the epilogue: each epilogue thread owns one token's accumulator row."""
+    top-k in the epilogue: each epilogue thread owns one token's accumulator row.
+
+    Every batch takes this one kernel.  A token whose k-th and next logits tie to fp32 rounding is routed by
+    the summation order, so a second kernel for some batch sizes would route it by the batch it is in."""
     from .expert import sm_count
     T, D = x.shape
     E = wr_kmajor.shape[0]

@@ -307,8 +307,8 @@ def test_padded_all_to_all_engine_repeats_without_memsets(dev, e_local, H, T, k,
                                      (9500, 200, 65, 8), (40, 4096, 256, 8),
                                      (4736, 64, 64, 8), (4737, 64, 64, 8)])
 def test_router_tile_edges(dev, T, D, E, k):
-    """Ragged 16-token tiles and last 64-element steps, expert passes of 8 to 64, and both sides of the
-    line to 128-token tiles (9472 tokens with 17 to 32 experts, 4736 with more)."""
+    """Batches around one 128-token tile's edges and of many tiles, last k-blocks of any length, and one to
+    sixteen 16-column steps of experts."""
     from iris_testing_b200.ops import cpu_ref, router_topk
     from iris_testing_b200.utils import gen_local_tokens, gen_router
     x = gen_local_tokens(1, T, D, torch.bfloat16, dev, 1, 0, "normal")
@@ -319,6 +319,20 @@ def test_router_tile_edges(dev, T, D, E, k):
     assert clear.float().mean() > 0.95
     assert torch.equal(idx[clear], ridx[clear])
     assert torch.allclose(w[clear], rw[clear], atol=1e-6, rtol=2e-4)      # fp32 sums of up to 4096 products
+
+
+@pytest.mark.parametrize("D,E,k,T", [(4096, 8, 2, 2400), (2048, 64, 8, 4800), (1024, 32, 2, 9600)])
+def test_a_token_is_routed_alike_in_every_batch(dev, D, E, k, T):
+    """Choices and weights of a token are the same bits whatever batch it comes in: near-ties of two logits
+    are decided by the summation order, which must not change with the number of tokens."""
+    from iris_testing_b200.ops import router_topk
+    from iris_testing_b200.utils import gen_local_tokens, gen_router
+    x = gen_local_tokens(1, T, D, torch.bfloat16, dev, 5, 0, "normal")
+    wr = gen_router(D, E, torch.bfloat16, dev, 5, std=None)
+    idx, w = router_topk(x, wr, k)
+    for n in (1, 17, 200, T // 2 - 64, T - 1):
+        i, v = router_topk(x[:n], wr, k)
+        assert torch.equal(i, idx[:n]) and torch.equal(v, w[:n]), n
 
 
 @pytest.mark.parametrize("n,E", [(0, 4), (1, 128), (1023, 3), (1024, 128), (1025, 1), (148 * 1024, 64),
