@@ -299,7 +299,7 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
             }
           }
           uint32_t* flag = reinterpret_cast<uint32_t*>(a.token_sync.p[peer]) + (a.mirror ? a.rank : e);
-          if (last) { if (peer == a.rank) red_add_relaxed_gpu(flag, 1u); else red_add_relaxed_sys(flag, 1u); }
+          if (last) red_add_relaxed_sys(flag, 1u);     // every rank adds to this word
         }
       }
     }
