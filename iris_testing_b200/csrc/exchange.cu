@@ -232,9 +232,8 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
     uint32_t* parts = a.parts + static_cast<size_t>(a.epoch & 1u) * a.parts_stride;
     uint32_t* next = a.parts + static_cast<size_t>(~a.epoch & 1u) * a.parts_stride;
     for (int i = blockIdx.x * blockDim.x + tid; i < a.parts_stride; i += gridDim.x * blockDim.x) next[i] = 0u;
-    __shared__ unsigned s_entered;
-    if (tid == 0) s_entered = a.mirror ? 0xffffffffu : 0u;
-    __syncthreads();
+    unsigned entered = a.mirror ? 0xffffffffu : 0u;   // peers seen to have entered: each thread's own copy, set after
+                                                      // a barrier, so that all threads of the block decide alike
     for (long long v = blockIdx.x; v < total * a.split; v += gridDim.x) {
       const long long u = v / a.split;
       const int share = static_cast<int>(v - u * a.split);
@@ -250,12 +249,12 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
       const int rows = min(a.block_m, n - m0);
       // A peer's buffers may be written once it has entered the epoch.  This rank's own rows may go at once (their
       // consumer ran earlier in this stream); only the count has to come after the flags were re-armed.
-      const bool need = !(s_entered >> peer & 1u);   // uniform for peers: their bits change between barriers
+      const bool need = !(entered >> peer & 1u);
       if (need && peer != a.rank) {
-        if (tid == 0 && wait_flag_geq(a.entered_local + peer, a.epoch, w, ST_TIMEOUT_BARRIER))
-          s_entered |= 1u << peer;
+        if (tid == 0) wait_flag_geq(a.entered_local + peer, a.epoch, w, ST_TIMEOUT_BARRIER);
         __syncthreads();
         if (s_abort) break;
+        entered |= 1u << peer;
       }
       const uint8_t* src;
       uint8_t* dst;
@@ -286,7 +285,7 @@ padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__
         bool ok = true;
         if (need && peer == a.rank) {
           ok = wait_flag_geq(a.entered_local + peer, a.epoch, w, ST_TIMEOUT_BARRIER);
-          if (ok) s_entered |= 1u << peer;
+          if (ok) entered |= 1u << peer;     // (only this thread asks)
         }
         if (ok) {
           if (peer == a.rank) fence_acq_rel_gpu(); else fence_acq_rel_sys();

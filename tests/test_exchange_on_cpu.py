@@ -197,3 +197,11 @@ def test_no_kernel_adds_to_a_flag_at_gpu_scope():
     """The same for every kernel, by the source: the counters in symmetric memory are added to by several ranks."""
     for f in sorted(CSRC.glob("*.cu*")):
         assert not re.search(r"red\.\w+\.gpu\b|red_add_\w+_gpu\b", f.read_text()), f.name
+
+
+@pytest.mark.parametrize("W,rank,EL,cap,split,blocks,mirror", CASES + [(8, 5, 2, 9, 2, 2, 0)])
+def test_threads_of_a_block_meet_at_the_same_barriers(exchange, W, rank, EL, cap, split, blocks, mirror):
+    """One thread waits for a peer on behalf of its block; whether the block waits must be decided alike by threads
+    that run ahead and threads that come late.  Rows, counts and flags land where they belong, none twice."""
+    r = exchange(W, rank, EL, cap, split, blocks, mirror)
+    assert r["diverged"] == 0 and r["wrong"] == 0 and r["status"] == 0, r
