@@ -165,8 +165,8 @@ struct PaddedArgs {
 };
 
 __global__ void __launch_bounds__(256, 4)
-padded_bulk_kernel(const uint8_t* __restrict__ src_rows, const int* __restrict__ counts,
-                   const int* __restrict__ dst_offsets, PaddedArgs a) {
+padded_bulk_kernel(const uint8_t* src_rows, const int* counts,
+                   const int* dst_offsets, PaddedArgs a) {
   extern __shared__ __align__(128) uint8_t a2a_smem[];
   __shared__ uint64_t bars[A2A_WARPS][2];
   __shared__ int s_abort;
@@ -408,14 +408,14 @@ __global__ void padded_wait_kernel(const int* pca, const uint32_t* counts_ready,
 // that pays, and more warps on the SM hide the index reads better.
 template <int KMAX, int U>   // KMAX: rows gathered at a time (any topk); U: 16-byte column pieces per lane
 __global__ void __launch_bounds__(256)
-weighted_gather_kernel(const __nv_bfloat16* __restrict__ ret_buf,
-                       const int* __restrict__ dst_slot,
-                       const int* __restrict__ topk_idx,
-                       const int* __restrict__ bucket_start,
-                       const float* __restrict__ topk_w, uint32_t* ret_sync,
-                       const int* __restrict__ send_counts, int T, int topk, int world,
+weighted_gather_kernel(const __nv_bfloat16* ret_buf,
+                       const int* dst_slot,
+                       const int* topk_idx,
+                       const int* bucket_start,
+                       const float* topk_w, uint32_t* ret_sync,
+                       const int* send_counts, int T, int topk, int world,
                        int e_local, int cap, int H, int block_m,
-                       __nv_bfloat16* __restrict__ y, int* status,
+                       __nv_bfloat16* y, int* status,
                        unsigned long long budget_ns, unsigned int* ticket) {
   __shared__ int s_abort;
   __shared__ int s_last;
@@ -442,11 +442,11 @@ weighted_gather_kernel(const __nv_bfloat16* __restrict__ ret_buf,
         wv[s] = 0.f;
         if (s0 + s < topk) {
           const int flat = t * topk + s0 + s;
-          const int ge = __ldg(topk_idx + flat);
-          const int m = __ldg(dst_slot + flat) - __ldg(bucket_start + ge);
+          const int ge = ld_32(topk_idx + flat);
+          const int m = ld_32(dst_slot + flat) - ld_32(bucket_start + ge);
           if (m < cap) {            // [dst, e] flattens to ge
             row[s] = reinterpret_cast<const uint4*>(ret_buf + (static_cast<size_t>(ge) * cap + m) * H);
-            wv[s] = __ldg(topk_w + flat);
+            wv[s] = ld_32(topk_w + flat);
           }
         }
       }
@@ -590,9 +590,9 @@ struct RetireArgs {
 // numbers, iteration, status) is read before or along with the first look at their counter.
 template <int KMAX>   // topk <= KMAX; about eight 16-byte loads per lane are kept in flight
 __global__ void __launch_bounds__(256, 4)
-slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __restrict__ dst_slot,
+slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* dst_slot,
                                    uint32_t* arrived, uint32_t expected, int T, int topk, int H,
-                                   __nv_bfloat16* __restrict__ y, RetireArgs ra, int* status,
+                                   __nv_bfloat16* y, RetireArgs ra, int* status,
                                    unsigned long long budget_ns, int wpt) {
   __shared__ int s_abort;
   __shared__ uint32_t s_iter;
@@ -605,7 +605,7 @@ slot_reduce_kernel(const __nv_bfloat16* out_slots, const int* __restrict__ dst_s
   auto find_rows = [&](int t) {
 #pragma unroll
     for (int s = 0; s < KMAX; ++s)
-      if (s < topk && t < T) next[s] = dst_slot != nullptr ? __ldg(dst_slot + t * topk + s) : t * topk + s;
+      if (s < topk && t < T) next[s] = dst_slot != nullptr ? ld_32(dst_slot + t * topk + s) : t * topk + s;
   };
   find_rows(warp / wpt);
   if (threadIdx.x == 32) s_iter = ra.iter_ptr != nullptr ? __ldcg(ra.iter_ptr) : 0u;

@@ -899,7 +899,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
         uint8_t* recv = reinterpret_cast<uint8_t*>(da.peer_recv[dst]);
         uint2* meta = reinterpret_cast<uint2*>(da.peer_meta[dst]);
         for (int p = p_lo + swarp; p < p_hi; p += SENDER_WARPS) {
-          const int flat = __ldg(da.send_order + send0 + p);
+          const int flat = ld_32(da.send_order + send0 + p);
           const int t = flat / da.topk;
           const int drow = drow0 + p;
           if (t < 0 || t >= da.num_tokens || drow >= da.cap_rows) {
@@ -912,7 +912,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
             uint4 v[8];
 #pragma unroll
             for (int j = 0; j < 8; ++j)
-              if (i + 32 * j < k16) v[j] = ld_nc_16(src + i + 32 * j);
+              if (i + 32 * j < k16) v[j] = ld_stream_16(src + i + 32 * j);
 #pragma unroll
             for (int j = 0; j < 8; ++j)
               if (i + 32 * j < k16) st_16(out + i + 32 * j, v[j]);
@@ -923,7 +923,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
             // position, so the rows of one (destination, expert) bucket return to consecutive
             // addresses (sequential remote writes) instead of to scattered token slots
             mv.x = (static_cast<uint32_t>(da.rank) << 24) | static_cast<uint32_t>(send0 + p);
-            mv.y = __float_as_uint(__ldg(da.topk_weight + flat));
+            mv.y = __float_as_uint(ld_32(da.topk_weight + flat));
             meta[drow] = mv;
           }
         }

@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sm100_ptx.cuh"
 #include "topk.cuh"
 
 namespace b200 {
@@ -43,7 +44,7 @@ struct RouterTile {
 
   // Logits of tokens [t0, t0 + TOK) (those below T) against all E experts into lg[TOK][E].
   // Every thread of the CTA takes part; ends with a barrier.
-  static __device__ __forceinline__ void logits(const __nv_bfloat16* __restrict__ x,
+  static __device__ __forceinline__ void logits(const __nv_bfloat16* x,
                                                 const __nv_bfloat16* __restrict__ wr_kmajor,
                                                 const float* __restrict__ bias, int T, int D, int E, int t0,
                                                 float* part, float* lg) {
@@ -75,7 +76,7 @@ struct RouterTile {
             const int i = (s0 + u * KS) * 8 + j * 4;
             const bool in = i + q < d16;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) xv[u][j][h] = in ? __ldg(xr[h] + i) : zero;
+            for (int h = 0; h < 2; ++h) xv[u][j][h] = in ? ld_16(xr[h] + i) : zero;
 #pragma unroll
             for (int n = 0; n < NT; ++n) wv[u][j][n] = in ? __ldg(wp + wo[n] + i) : zero;
           }

@@ -242,8 +242,8 @@ constexpr int PLAN_SUB = 1024;       // copies per pass of a CTA
 constexpr int PLAN_MAX_CHUNKS = 148;
 
 __global__ void __launch_bounds__(PLAN_THREADS)
-plan_count_kernel(const int* __restrict__ topk_idx, int n_flat, int num_experts, int chunk,
-                  int* __restrict__ rank_in_bucket, int* __restrict__ hist) {
+plan_count_kernel(const int* topk_idx, int n_flat, int num_experts, int chunk,
+                  int* rank_in_bucket, int* hist) {
   constexpr int WARPS = PLAN_THREADS / 32, PER = PLAN_SUB / PLAN_THREADS;
   __shared__ int s_cnt[WARPS][B200_MAX_EXPERTS];
   __shared__ int s_run[B200_MAX_EXPERTS];
@@ -258,7 +258,7 @@ plan_count_kernel(const int* __restrict__ topk_idx, int n_flat, int num_experts,
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       const int i = base + (warp * PER + j) * 32 + lane;
-      ev[j] = i < hi ? topk_idx[i] : -1;
+      ev[j] = i < hi ? ld_32(topk_idx + i) : -1;
       if (ev[j] >= num_experts) ev[j] = -1;
       if (ev[j] < 0) ev[j] = -1;
     }
@@ -289,9 +289,9 @@ plan_count_kernel(const int* __restrict__ topk_idx, int n_flat, int num_experts,
 }
 
 __global__ void __launch_bounds__(PLAN_THREADS)
-plan_place_kernel(const int* __restrict__ topk_idx, int* __restrict__ rank_in_bucket, const int* __restrict__ hist,
-                  int n_flat, int num_experts, int chunk, int* __restrict__ counts, int* __restrict__ bucket_start,
-                  int* __restrict__ send_order, int* __restrict__ dst_slot, PlanPushArgs push, int do_push) {
+plan_place_kernel(const int* topk_idx, int* rank_in_bucket, const int* hist,
+                  int n_flat, int num_experts, int chunk, int* counts, int* bucket_start,
+                  int* send_order, int* dst_slot, PlanPushArgs push, int do_push) {
   __shared__ int s_tot[B200_MAX_EXPERTS];
   __shared__ int s_before[B200_MAX_EXPERTS];      // copies of the expert in earlier chunks
   __shared__ int s_start[B200_MAX_EXPERTS + 1];
@@ -309,7 +309,7 @@ plan_place_kernel(const int* __restrict__ topk_idx, int* __restrict__ rank_in_bu
   for (int e = warp; e < num_experts; e += PLAN_THREADS / 32) {
     int before = 0, tot = 0;
     for (int c = lane; c < chunks; c += 32) {
-      const int v = hist[e * chunks + c];
+      const int v = ld_32(hist + e * chunks + c);
       tot += v;
       if (c < me) before += v;
     }
@@ -333,9 +333,9 @@ plan_place_kernel(const int* __restrict__ topk_idx, int* __restrict__ rank_in_bu
   }
   const int hi = min(n_flat, (me + 1) * chunk);
   for (int i = me * chunk + tid; i < hi; i += PLAN_THREADS) {
-    const int e = topk_idx[i];
+    const int e = ld_32(topk_idx + i);
     if (e < 0 || e >= num_experts) continue;
-    const int rank = s_before[e] + rank_in_bucket[i];
+    const int rank = s_before[e] + ld_32(rank_in_bucket + i);
     const int pos = s_start[e] + rank;
     rank_in_bucket[i] = rank;
     send_order[pos] = i;
@@ -382,11 +382,11 @@ constexpr int SMALL_MAX_FLAT = 4096;
 
 template <int NT, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32, 1)
-route_plan_small_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wr_kmajor,
+route_plan_small_kernel(const __nv_bfloat16* x, const __nv_bfloat16* __restrict__ wr_kmajor,
                         const float* __restrict__ bias, int T, int D, int E, int k, int renorm,
-                        int* __restrict__ topk_idx, float* __restrict__ topk_w, int* __restrict__ counts,
-                        int* __restrict__ bucket_start, int* __restrict__ send_order,
-                        int* __restrict__ dst_slot, PlanPushArgs push, int do_push, unsigned int* ticket) {
+                        int* topk_idx, float* topk_w, int* counts,
+                        int* bucket_start, int* send_order,
+                        int* dst_slot, PlanPushArgs push, int do_push, unsigned int* ticket) {
   constexpr int THREADS = WARPS * 32;
   constexpr int SEG = SMALL_MAX_FLAT / WARPS;      // most copies of one warp's segment
   extern __shared__ __align__(16) float router_smem[];

@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <stdint.h>
+#include <string.h>
 
 namespace b200 {
 
@@ -94,7 +95,19 @@ __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async;" ::: "memory");
 }
 
-// 16-byte vector copy helpers (global).
+// Global loads and stores.  ld_nc_16 (like __ldg and const __restrict__) is for memory that no kernel writes during the
+// caller's lifetime, which in a chained launch begins before the predecessor's last write; ld_32, ld_16 and
+// ld_stream_16 (not kept in L1) are ordinary loads, which chain_wait() holds back and makes the predecessor's writes
+// visible to.
+template <typename T>
+__device__ __forceinline__ T ld_32(const T* p) {
+  static_assert(sizeof(T) == 4, "one 32-bit word");
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+  T t;
+  memcpy(&t, &v, 4);
+  return t;
+}
 __device__ __forceinline__ uint4 ld_nc_16(const void* p) {
   uint4 v;
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
@@ -105,6 +118,14 @@ __device__ __forceinline__ uint4 ld_nc_16(const void* p) {
 __device__ __forceinline__ uint4 ld_16(const void* p) {
   uint4 v;
   asm volatile("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ uint4 ld_stream_16(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p)
                : "memory");
@@ -210,7 +231,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, WaitCt
 // start wherever there is room: at once where that kernel runs one CTA per SM or only a few CTAs, at the
 // end where it is a grid of many small CTAs, which would pile up on the first SMs to come free (24 us
 // instead of 18 us for the slot reduction of 3000 tokens).  Both are no-ops in a kernel that was
-// launched the ordinary way.
+// launched the ordinary way.  What an earlier kernel of a chain wrote is read by ordinary loads only (see ld_32).
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void chain_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
