@@ -433,7 +433,7 @@ weighted_gather_kernel(const __nv_bfloat16* ret_buf,
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int t = warp; t < T && !s_abort; t += nwarps) {
-    const uint4* row[KMAX];        // null: no such slot, or dropped by capacity
+    const uint4* row[KMAX];        // null: no such slot, no expert, or dropped by capacity
     float wv[KMAX];
     auto find = [&](int s0) {
 #pragma unroll
@@ -443,8 +443,9 @@ weighted_gather_kernel(const __nv_bfloat16* ret_buf,
         if (s0 + s < topk) {
           const int flat = t * topk + s0 + s;
           const int ge = ld_32(topk_idx + flat);
+          if (ge < 0 || ge >= world * e_local) continue;
           const int m = ld_32(dst_slot + flat) - ld_32(bucket_start + ge);
-          if (m < cap) {            // [dst, e] flattens to ge
+          if (m >= 0 && m < cap) {  // [dst, e] flattens to ge
             row[s] = reinterpret_cast<const uint4*>(ret_buf + (static_cast<size_t>(ge) * cap + m) * H);
             wv[s] = ld_32(topk_w + flat);
           }

@@ -16,6 +16,8 @@
 //   bucket_start [num_experts + 1]  exclusive scan of counts
 //   send_order   [n_flat]           flat (token*k+slot) ids sorted by expert, stable
 //   dst_slot     [n_flat]           inverse of send_order (may be null)
+// Copies without an expert (ids outside [0, num_experts)) get no place: -1 in dst_slot
+// and behind the last row of send_order.
 // The caller passes inputs and outputs only.
 //
 // Limit: n_flat <= B200_PLAN_NOALLOC_MAX (1 048 576 routed copies, a 4 MiB

@@ -143,7 +143,8 @@ __global__ void plan_rank_kernel(const int* __restrict__ topk_idx, int n_flat, i
 
 // ---------------------------------------------------------------------------
 // Plan, step 2: bucket offsets (exclusive scan over experts), the packed send
-// order, and -- when `peer_counts` is given -- the push of this rank's counts
+// order (copies without an expert get no place: -1 in dst_slot, -1 behind the
+// last row), and -- when `peer_counts` is given -- the push of this rank's counts
 // row to every rank followed by an epoch-stamped flag.  Before touching a
 // peer's tables the kernel checks that the peer has retired the iteration that
 // last used the same parity slot.
@@ -280,7 +281,7 @@ plan_count_kernel(const int* topk_idx, int n_flat, int num_experts, int chunk,
 #pragma unroll
     for (int j = 0; j < PER; ++j) {
       const int i = base + (warp * PER + j) * 32 + lane;
-      if (ev[j] >= 0) rank_in_bucket[i] = s_cnt[warp][ev[j]] + r[j];
+      if (i < hi) rank_in_bucket[i] = ev[j] >= 0 ? s_cnt[warp][ev[j]] + r[j] : -1;
     }
     __syncthreads();
   }
@@ -334,7 +335,11 @@ plan_place_kernel(const int* topk_idx, int* rank_in_bucket, const int* hist,
   const int hi = min(n_flat, (me + 1) * chunk);
   for (int i = me * chunk + tid; i < hi; i += PLAN_THREADS) {
     const int e = ld_32(topk_idx + i);
-    if (e < 0 || e >= num_experts) continue;
+    if (i >= s_start[num_experts]) send_order[i] = -1;
+    if (e < 0 || e >= num_experts) {
+      if (dst_slot) dst_slot[i] = -1;
+      continue;
+    }
     const int rank = s_before[e] + ld_32(rank_in_bucket + i);
     const int pos = s_start[e] + rank;
     rank_in_bucket[i] = rank;
@@ -363,7 +368,11 @@ __global__ void plan_finalize_kernel(const int* __restrict__ topk_idx,
   }
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_flat; i += gridDim.x * blockDim.x) {
     const int e = topk_idx[i];
-    if (e < 0 || e >= num_experts) continue;
+    if (i >= s_start[num_experts]) send_order[i] = -1;
+    if (e < 0 || e >= num_experts) {
+      if (dst_slot) dst_slot[i] = -1;
+      continue;
+    }
     const int pos = s_start[e] + rank_in_bucket[i];
     send_order[pos] = i;
     if (dst_slot) dst_slot[i] = pos;
@@ -531,16 +540,16 @@ __global__ void capacity_kernel(const int* __restrict__ send_counts, CapacityArg
   if (tid < 4) out[tid] = s_red[tid];
 }
 
-// Gathers the packed send payload: payload[j, :] = x[send_order[j] / topk, :].
+// Gathers the packed send payload: payload[j, :] = x[send_order[j] / topk, :]; zero where send_order is -1.
 __global__ void pack_rows_kernel(const uint4* __restrict__ x, const int* __restrict__ send_order,
                                  int n_flat, int topk, int row16, uint4* __restrict__ payload) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   for (int j = warp; j < n_flat; j += nwarps) {
-    const int t = send_order[j] / topk;
-    const uint4* src = x + static_cast<size_t>(t) * row16;
+    const int flat = send_order[j];
+    const uint4* src = x + static_cast<size_t>(max(flat, 0) / topk) * row16;
     uint4* dst = payload + static_cast<size_t>(j) * row16;
-    for (int i = lane; i < row16; i += 32) dst[i] = ld_nc_16(src + i);
+    for (int i = lane; i < row16; i += 32) dst[i] = flat >= 0 ? ld_nc_16(src + i) : make_uint4(0u, 0u, 0u, 0u);
   }
 }
 

@@ -49,7 +49,8 @@ def weighted_gather(ret_buf: torch.Tensor, plan, topk_idx: torch.Tensor, topk_w:
                     ret_sync: Optional[torch.Tensor], world: int, capacity: int,
                     status: Optional[torch.Tensor] = None, wait_budget_ms: float = 2000.0,
                     rearm_ticket: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """y[t] = sum_slot topk_w[t, slot] * ret_buf[cell of (t, slot)]   -> [T, H].
+    """y[t] = sum_slot topk_w[t, slot] * ret_buf[cell of (t, slot)]   -> [T, H].  Slots without an expert (outside
+    ``[0, world * e_local)``) and rows dropped by the capacity take no part.
 
     ``plan`` is the :class:`~iris_testing_b200.ops.plan.Plan` used for the dispatch.  On CUDA
     the kernel first waits (bounded) until ``ret_sync`` shows every returned tile; with
@@ -60,10 +61,12 @@ def weighted_gather(ret_buf: torch.Tensor, plan, topk_idx: torch.Tensor, topk_w:
     e_local = ret_buf.shape[1]
     if not ret_buf.is_cuda:
         flat_e = topk_idx.reshape(-1).long()
+        keep = (flat_e >= 0) & (flat_e < world * e_local)
+        flat_e = flat_e.clamp(0, world * e_local - 1)
         m = plan.dst_slot.long() - plan.bucket_start.long()[flat_e]
-        keep = (m < capacity)
-        rows = ret_buf.reshape(-1, H)[(flat_e * capacity + m.clamp(max=capacity - 1))].float()
-        rows = rows * (topk_w.reshape(-1, 1).float() * keep.unsqueeze(1))
+        keep &= (m >= 0) & (m < capacity)
+        rows = ret_buf.reshape(-1, H)[(flat_e * capacity + m.clamp(0, capacity - 1))].float()
+        rows = (rows * topk_w.reshape(-1, 1).float()).masked_fill(~keep.unsqueeze(1), 0.0)
         return rows.view(T, k, H).sum(dim=1).to(ret_buf.dtype)
     fn = declare("b200_weighted_gather",
                  [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,

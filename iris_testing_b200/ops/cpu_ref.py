@@ -46,23 +46,32 @@ class PlanRef:
 
 
 def plan_ref(topk_idx: torch.Tensor, num_experts: int) -> PlanRef:
-    """Bucket every routed copy by expert, keeping (token, slot) order inside a bucket."""
+    """Bucket every routed copy by expert, keeping (token, slot) order inside a bucket.  Copies without an
+    expert (numbers outside ``[0, num_experts)``) are dropped: -1 in dst_slot and rank_in_bucket, and behind the
+    last row of send_order."""
     flat = topk_idx.reshape(-1).to(torch.int64)
-    n = flat.numel()
-    counts = torch.bincount(flat, minlength=num_experts)[:num_experts]
-    start = torch.zeros(num_experts + 1, dtype=torch.int64, device=flat.device)
+    n, dev = flat.numel(), flat.device
+    kept = torch.nonzero((flat >= 0) & (flat < num_experts)).reshape(-1)
+    counts = torch.bincount(flat[kept], minlength=num_experts)
+    start = torch.zeros(num_experts + 1, dtype=torch.int64, device=dev)
     start[1:] = torch.cumsum(counts, 0)
-    order = torch.sort(flat, stable=True).indices
-    dst_slot = torch.empty(n, dtype=torch.int64, device=flat.device)
-    dst_slot[order] = torch.arange(n, device=flat.device)
-    rank = dst_slot - start[flat]
+    order = torch.full((n,), -1, dtype=torch.int64, device=dev)
+    order[:kept.numel()] = kept[torch.sort(flat[kept], stable=True).indices]
+    dst_slot = torch.full((n,), -1, dtype=torch.int64, device=dev)
+    dst_slot[order[:kept.numel()]] = torch.arange(kept.numel(), device=dev)
+    rank = torch.full((n,), -1, dtype=torch.int64, device=dev)
+    rank[kept] = dst_slot[kept] - start[flat[kept]]
     i32 = torch.int32
     return PlanRef(counts.to(i32), start.to(i32), order.to(i32), dst_slot.to(i32), rank.to(i32))
 
 
 def pack_ref(x: torch.Tensor, send_order: torch.Tensor, topk: int) -> torch.Tensor:
-    """payload[j] = x[send_order[j] // topk] (a token routed to k experts appears k times)."""
-    return x[(send_order.long() // topk)]
+    """payload[j] = x[send_order[j] // topk] (a token routed to k experts appears k times); zero where
+    send_order is -1."""
+    order = send_order.long()
+    if x.shape[0] == 0 or order.numel() == 0:
+        return x.new_zeros((order.numel(), x.shape[1]))
+    return x[order.clamp(min=0) // topk].masked_fill((order < 0).unsqueeze(1), 0)
 
 
 def expert_offsets_ref(send_counts: torch.Tensor) -> torch.Tensor:

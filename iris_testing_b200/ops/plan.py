@@ -58,7 +58,9 @@ def plan_workspace(num_experts: int, device) -> torch.Tensor:
 
 def make_plan(topk_idx: torch.Tensor, num_experts: int, out: Optional[Plan] = None,
               push: Optional[PlanPushArgs] = None, workspace: Optional[torch.Tensor] = None) -> Plan:
-    """topk_idx int32 [T, k] (global expert ids) -> :class:`Plan`.
+    """topk_idx int32 [T, k] (global expert ids) -> :class:`Plan`.  Copies without an expert (ids outside
+    ``[0, num_experts)``: the router's -1 for a NaN token or masked experts) are dropped: -1 in ``dst_slot`` and
+    ``rank_in_bucket``, and behind the last row of ``send_order``.
 
     ``out`` and ``workspace`` (:func:`plan_workspace`) let a caller reuse preallocated buffers; ``push`` (fused engine only)
     makes the second kernel also publish the counts to every peer.
@@ -85,7 +87,8 @@ def make_plan(topk_idx: torch.Tensor, num_experts: int, out: Optional[Plan] = No
 
 
 def pack_rows(x: torch.Tensor, send_order: torch.Tensor, topk: int) -> torch.Tensor:
-    """payload[j] = x[send_order[j] // topk]: the packed send payload (dst-major, expert-major)."""
+    """payload[j] = x[send_order[j] // topk]: the packed send payload (dst-major, expert-major); zero
+    where ``send_order`` is -1."""
     if not use_native(x):
         return cpu_ref.pack_ref(x, send_order, topk)
     require(x.is_contiguous() and x.shape[1] % 8 == 0 and x.element_size() == 2,

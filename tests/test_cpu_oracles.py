@@ -259,3 +259,27 @@ def test_small_token_path_rule():
     assert tiny.uses_small_path(64) and tiny.uses_small_path(2048) and not tiny.uses_small_path(2049)
     mixtral.small_path = False
     assert not mixtral.uses_small_path(64) and mixtral.launches_for(64) == 6
+
+
+def test_copies_routed_to_no_expert_are_dropped():
+    """Expert -1 (fewer than k logits above -inf: NaN tokens, masked experts) or one past the last: the copy gets no
+    place (-1), the send order ends with -1, its payload row is zero and the weighted sum leaves it out."""
+    from iris_testing_b200.ops import cpu_ref, make_plan
+    from iris_testing_b200.ops.combine import weighted_gather
+    from iris_testing_b200.ops.plan import pack_rows
+    idx = torch.tensor([[2, 0], [-1, 1], [0, 4], [1, -1], [-1, -1]], dtype=torch.int32)
+    p = make_plan(idx, 4)
+    assert p.counts.tolist() == [2, 2, 1, 0] and p.bucket_start.tolist() == [0, 2, 4, 5, 5]
+    assert p.send_order.tolist() == [1, 4, 3, 6, 0, -1, -1, -1, -1, -1]
+    assert p.dst_slot.tolist() == [4, 0, -1, 2, 1, -1, 3, -1, -1, -1]
+    assert p.rank_in_bucket.tolist() == [0, 0, -1, 0, 1, -1, 1, -1, -1, -1]
+    x = torch.arange(1, 41, dtype=torch.float32).view(5, 8)
+    rows = pack_rows(x, p.send_order, 2)
+    assert torch.equal(rows[:5], x[[0, 2, 1, 3, 0]]) and int(rows[5:].abs().sum()) == 0
+    ret = torch.zeros(1, 4, 2, 8)
+    for e in range(4):
+        n = int(p.counts[e])
+        ret[0, e, :n] = rows[int(p.bucket_start[e]):int(p.bucket_start[e]) + n]
+    w = torch.tensor([[0.5, 0.25], [float("nan"), 1.0], [2.0, 3.0], [1.0, 7.0], [float("nan"), 1.0]])
+    y = weighted_gather(ret, p, idx, w, None, 1, 2)
+    assert torch.equal(y, x * torch.tensor([0.75, 1.0, 2.0, 1.0, 0.0]).view(5, 1))

@@ -347,6 +347,76 @@ def test_plan_chunk_edges(dev, n, E):
         assert torch.equal(getattr(p, name), getattr(r, name)), name
 
 
+@pytest.mark.parametrize("T,k,E", [(1, 1, 1), (5, 2, 4), (600, 3, 8), (40000, 4, 128)])
+def test_plan_and_its_users_drop_copies_without_an_expert(dev, T, k, E):
+    """Expert numbers below zero and past the last: no place for the copy, -1 behind the send order's last row, a zero
+    payload row, no part in the weighted sum; with none left at all too.  Both plan entry points."""
+    from iris_testing_b200 import _native as nv
+    from iris_testing_b200.ops import cpu_ref, make_plan
+    from iris_testing_b200.ops._common import ptr, stream_ptr
+    from iris_testing_b200.ops.combine import weighted_gather
+    from iris_testing_b200.ops.plan import pack_rows
+    g = torch.Generator(device="cpu").manual_seed(T + E)
+    H = 72
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).to(dev)
+    for lo, hi in ((-1, E), (-3, E + 3), (-1, 0)):
+        idx = torch.randint(lo, hi, (T, k), generator=g, dtype=torch.int32).to(dev)
+        p, r = make_plan(idx, E), cpu_ref.plan_ref(idx, E)
+        for name in ("counts", "bucket_start", "send_order", "dst_slot", "rank_in_bucket"):
+            assert torch.equal(getattr(p, name), getattr(r, name)), name
+        q = {n: torch.full_like(getattr(r, n), 12345) for n in ("counts", "bucket_start", "send_order", "dst_slot")}
+        assert nv.lib().b200_plan_noalloc(ptr(idx), T * k, E, *(ptr(t) for t in q.values()), stream_ptr(idx)) == 0
+        for name, t in q.items():
+            assert torch.equal(t, getattr(r, name)), name
+        payload = pack_rows(x, p.send_order, k)
+        assert torch.equal(payload, cpu_ref.pack_ref(x, r.send_order, k))
+        cap = max(int(p.counts.max()), 1)
+        ret = torch.zeros(1, E, cap, H, dtype=torch.bfloat16, device=dev)
+        for e, (a, n) in enumerate(zip(p.bucket_start.tolist(), p.counts.tolist())):
+            ret[0, e, :n] = payload[a:a + n]
+        keep = (idx >= 0) & (idx < E)
+        w = torch.where(keep, torch.rand(T, k, generator=g).to(dev), float("nan"))
+        y = weighted_gather(ret, p, idx, w, None, 1, cap)
+        sums = torch.where(keep, w, 0.0).double().sum(1, keepdim=True)
+        mag = x.double().abs() * sums                    # bf16 rounding, fp32 sums of k products
+        assert bool(((y.double() - x.double() * sums).abs() <= mag * (2.0 ** -8 + k * 2.0 ** -22)).all())
+
+
+def test_a_token_of_nan_disturbs_no_other(dev):
+    """Route, pack, dispatch, return and weighted sum with NaN tokens and masked experts: their copies are dropped and
+    every other token comes back as it would alone."""
+    from iris_testing_b200.ops import router_topk
+    from iris_testing_b200.parallel.padded_a2a import PaddedAllToAll
+    from iris_testing_b200.parallel.symm import SymmetricHeap
+    from iris_testing_b200.utils import gen_local_tokens, gen_router, route_and_pack
+    T, H, E, k = 300, 136, 8, 2
+    x = gen_local_tokens(1, T, H, torch.bfloat16, dev, 1, 0, "normal")
+    router = gen_router(H, E, torch.bfloat16, dev, 3, std=None)
+    clean_idx, clean_w = router_topk(x, router, k)
+    bad = torch.zeros(T, dtype=torch.bool, device=dev)
+    bad[::7] = True
+    x[bad] = float("nan")
+    payload, counts, dst_off, _, idx, wgt, plan = route_and_pack(x, router, k, 1, E)
+    assert bool((idx[bad] == -1).all()) and torch.equal(idx[~bad], clean_idx[~bad]) and torch.equal(wgt[~bad], clean_w[~bad])
+    assert int(counts.sum()) == int((~bad).sum()) * k and bool(torch.isfinite(payload).all())
+    heap = SymmetricHeap(2 * E * T * H * 2 + (32 << 20))
+    a2a = PaddedAllToAll(heap, E, T, H, torch.bfloat16, with_return=True)
+    a2a.dispatch(payload, counts, dst_off)
+    a2a.wait()
+    a2a.send_back()
+    y = a2a.reduce(plan, idx, wgt)
+    heap.check_status()
+    ref = x.double() * wgt.double().sum(1, keepdim=True)
+    assert int(y[bad].abs().sum()) == 0
+    assert bool(((y.double() - ref).abs()[~bad] <= ref.abs()[~bad] * (2.0 ** -8 + k * 2.0 ** -22)).all())
+    bias = torch.full((E,), -float("inf"), device=dev)
+    bias[5] = 0.0                                        # one expert left of two asked for
+    idx, wgt = router_topk(x[~bad], router, k, bias=bias)
+    assert bool((idx == torch.tensor([5, -1], device=dev)).all()) and bool((wgt == torch.tensor([1.0, 0.0], device=dev)).all())
+    del a2a
+    heap.close()
+
+
 @pytest.mark.parametrize("G,K,N", [(1, 8, 8), (2, 64, 64), (3, 72, 200), (2, 136, 56), (32, 768, 768)])
 def test_weight_transpose_kernel(dev, G, K, N):
     from iris_testing_b200.ops.expert import _to_kmajor_cuda as to_kmajor
