@@ -650,8 +650,10 @@ extern "C" int b200_route_plan_small(const void* x, const void* wr_kmajor, const
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(wr_kmajor)) & 15u) != 0) return -3;
   b200::PlanPushArgs pz;
   memset(&pz, 0, sizeof(pz));
-  auto go = [&](auto kern, int threads, int smem) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  // The limit belongs to the kernel, not to the launch: every call sets the same one, or a call from another thread
+  // with fewer experts could lower it between another's setting and launch.
+  auto go = [&](auto kern, int threads, int smem, int limit) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
     if (e != cudaSuccess) return static_cast<int>(e);
     e = b200::launch_chained(kern, dim3(std::max(1, (T + 15) / 16)), dim3(threads), smem,
                              static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x),
@@ -661,7 +663,8 @@ extern "C" int b200_route_plan_small(const void* x, const void* wr_kmajor, const
     return static_cast<int>(e);
   };
 #define B200_SMALL(NT, WARPS) \
-  go(b200::route_plan_small_kernel<NT, WARPS>, WARPS * 32, b200::RouterTile<NT, WARPS>::smem_bytes(E))
+  go(b200::route_plan_small_kernel<NT, WARPS>, WARPS * 32, b200::RouterTile<NT, WARPS>::smem_bytes(E), \
+     b200::RouterTile<NT, WARPS>::smem_bytes(B200_MAX_EXPERTS))
   if (E <= 8) return B200_SMALL(1, 16);
   if (E <= 16) return B200_SMALL(2, 16);
   if (E <= 32) return B200_SMALL(4, 16);

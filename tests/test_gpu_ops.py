@@ -335,6 +335,54 @@ def test_a_token_is_routed_alike_in_every_batch(dev, D, E, k, T):
         assert torch.equal(i, idx[:n]) and torch.equal(v, w[:n]), n
 
 
+def test_small_route_and_plan_from_several_threads(dev):
+    """Host threads with other numbers of experts in the same kernel: no launch is refused and every result is that
+    of the call alone."""
+    import ctypes as C
+    import threading
+    from iris_testing_b200.ops import cpu_ref
+    from iris_testing_b200.ops._common import declare
+    from iris_testing_b200.ops.plan import PlanPushArgs
+    from iris_testing_b200.ops.router import router_kmajor
+    from iris_testing_b200.utils import gen_local_tokens, gen_router
+    fn = declare("b200_route_plan_small",
+                 [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
+                  C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(PlanPushArgs), C.c_void_p, C.c_void_p])
+    T, D, k, errors = 48, 64, 2, []
+
+    def work(E):
+        i32 = dict(dtype=torch.int32, device=dev)
+        x = gen_local_tokens(1, T, D, torch.bfloat16, dev, E, 0, "normal")
+        wr = gen_router(D, E, torch.bfloat16, dev, E, std=None)
+        wk = router_kmajor(wr)
+        idx, w = torch.empty(T, k, **i32), torch.empty(T, k, dtype=torch.float32, device=dev)
+        outs = [torch.empty(n, **i32) for n in (E, E + 1, T * k, T * k)]
+        ticket = torch.zeros(1, **i32)
+        stream = torch.cuda.Stream(dev)
+        torch.cuda.synchronize()
+        for _ in range(2000):
+            rc = fn(x.data_ptr(), wk.data_ptr(), None, T, D, E, k, 0, idx.data_ptr(), w.data_ptr(),
+                    *(t.data_ptr() for t in outs), None, ticket.data_ptr(), stream.cuda_stream)
+            if rc != 0:
+                errors.append((E, rc))
+                break
+        stream.synchronize()
+        ref = cpu_ref.router_topk_ref(x, wr, k)[0]
+        plan = cpu_ref.plan_ref(idx, E)
+        clear = cpu_ref.clear_routing_mask(x, wr, k, None)
+        if not errors and not (torch.equal(idx[clear], ref[clear]) and torch.equal(outs[0], plan.counts)
+                               and torch.equal(outs[2], plan.send_order) and torch.equal(outs[3], plan.dst_slot)):
+            errors.append((E, "wrong"))
+
+    work(40), work(128)                                  # settled before the threads start
+    threads = [threading.Thread(target=work, args=(E,)) for E in (40, 128, 64)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+
+
 @pytest.mark.parametrize("n,E", [(0, 4), (1, 128), (1023, 3), (1024, 128), (1025, 1), (148 * 1024, 64),
                                  (148 * 1024 + 1, 128), (400000, 8)])
 def test_plan_chunk_edges(dev, n, E):
