@@ -227,7 +227,7 @@ class MoELayer(nn.Module):
         pair = cfg.cta_pair
         if os.getenv("B200MOE_CTA_PAIR", "") in ("0", "1"):       # override for tile-shape experiments
             pair = os.environ["B200MOE_CTA_PAIR"] == "1"
-        self._cta_pair = pair                       # None: per call, by the rows per expert
+        self._cta_pair = pair                       # None: by the rows per expert (_uses_pairs)
         self._budget_ns = int(cfg.wait_budget_ms * 1e6)
         self.recv = self.meta = self.ready = self.hidden = None
         self._alloc_capacity(cap)
@@ -386,12 +386,17 @@ class MoELayer(nn.Module):
         return (1 if self.uses_small_path(T) else 3) + (2 if self.cfg.gated else 1) + 1
 
     def _uses_pairs(self, T: int) -> int:
-        """1 when the GEMM kernels of a forward of ``T`` tokens run on CTA pairs (256-row tiles)."""
+        """1 when the GEMM kernels of a forward of ``T`` tokens run on CTA pairs (256-row tiles).
+
+        With several ranks an expert's rows come from all of them and this rank knows its own batch only: a short batch
+        here says nothing about the long ones of its peers, so the layer's ``max_tokens``, which all ranks share,
+        decides there."""
         cfg = self.cfg
         if self._cta_pair is not None:
             return int(bool(self._cta_pair))
-        rows = T * cfg.topk * cfg.world_size / cfg.num_experts
-        return int(rows >= 128 if any(self.wide_tiles) else pairs_pay(rows))
+        alone = cfg.world_size == 1
+        rows = (T if alone else self.max_tokens) * cfg.topk * cfg.world_size / cfg.num_experts
+        return int(pairs_pay(rows) if alone and not any(self.wide_tiles) else rows >= 128)
 
     @property
     def launches_per_forward(self) -> int:

@@ -283,3 +283,26 @@ def test_copies_routed_to_no_expert_are_dropped():
     w = torch.tensor([[0.5, 0.25], [float("nan"), 1.0], [2.0, 3.0], [1.0, 7.0], [float("nan"), 1.0]])
     y = weighted_gather(ret, p, idx, w, None, 1, 2)
     assert torch.equal(y, x * torch.tensor([0.75, 1.0, 2.0, 1.0, 0.0]).view(5, 1))
+
+
+def test_tile_geometry_rule():
+    """One rank: by the rows per expert of each call.  Several ranks: by max_tokens, whatever this rank's batch (its
+    experts receive the peers' rows too), and alike on every rank."""
+    from iris_testing_b200.config import MoEConfig
+    from iris_testing_b200.models import MoELayer
+
+    def layer(world, max_tokens, pair=None):
+        class Rule:
+            _uses_pairs = MoELayer._uses_pairs
+        r = Rule()
+        r.cfg = MoEConfig(hidden_dim=64, ffn_dim=128, num_experts=8, topk=2, world_size=world)
+        r.max_tokens, r.wide_tiles, r._cta_pair = max_tokens, (0, 0), pair
+        return r
+
+    one = layer(1, 16384)
+    assert [one._uses_pairs(T) for T in (64, 511, 512, 1024, 1025, 1408, 1409, 16384)] == [0, 0, 1, 1, 0, 0, 1, 1]
+    for T in (0, 1, 64, 300, 2048):
+        assert layer(8, 2048)._uses_pairs(T) == 1              # 4096 rows per expert when all ranks are full
+        assert layer(8, 63)._uses_pairs(min(T, 63)) == 0       # 126 rows
+        assert layer(2, 256)._uses_pairs(min(T, 256)) == 1     # 128 rows
+    assert layer(8, 2048, pair=False)._uses_pairs(2048) == 0 and layer(1, 64, pair=True)._uses_pairs(1) == 1
