@@ -50,10 +50,14 @@ def _plan_fn():
                                     C.c_void_p, C.c_void_p, C.c_void_p, C.POINTER(PlanPushArgs), C.c_void_p])
 
 
+def _workspace_ints(num_experts: int) -> int:
+    return declare("b200_plan_ws_ints", [C.c_int])(num_experts)
+
+
 def plan_workspace(num_experts: int, device) -> torch.Tensor:
     """Scratch of the plan kernels for lists of any length (contents irrelevant between calls; calls that
     may overlap need separate ones)."""
-    return torch.empty(declare("b200_plan_ws_ints", [C.c_int])(num_experts), dtype=torch.int32, device=device)
+    return torch.empty(_workspace_ints(num_experts), dtype=torch.int32, device=device)
 
 
 def make_plan(topk_idx: torch.Tensor, num_experts: int, out: Optional[Plan] = None,
@@ -78,6 +82,8 @@ def make_plan(topk_idx: torch.Tensor, num_experts: int, out: Optional[Plan] = No
                    torch.empty(n, **i32), torch.empty(n, **i32), torch.empty(n, **i32))
     idx = topk_idx if topk_idx.is_contiguous() else topk_idx.contiguous()
     ws = workspace if workspace is not None else plan_workspace(num_experts, dev)
+    require(ws.dtype == torch.int32 and ws.is_contiguous() and ws.numel() >= _workspace_ints(num_experts),
+            "workspace must be plan_workspace(num_experts, device) of at least as many experts")
     rc = _plan_fn()(ptr(idx), n, num_experts, ptr(out.rank_in_bucket), ptr(out.counts),
                     ptr(out.bucket_start), ptr(out.send_order), ptr(out.dst_slot), ptr(ws),
                     C.byref(push) if push is not None else None, stream_ptr(idx))

@@ -395,6 +395,15 @@ def test_plan_chunk_edges(dev, n, E):
         assert torch.equal(getattr(p, name), getattr(r, name)), name
 
 
+def test_plan_refuses_a_short_workspace(dev):
+    from iris_testing_b200.ops import make_plan
+    from iris_testing_b200.ops.plan import plan_workspace
+    idx = torch.zeros((4, 2), dtype=torch.int32, device=dev)
+    with pytest.raises(ValueError, match="workspace"):
+        make_plan(idx, 16, workspace=plan_workspace(8, dev))
+    assert make_plan(idx, 8, workspace=plan_workspace(16, dev)).counts.tolist() == [8] + [0] * 7
+
+
 @pytest.mark.parametrize("T,k,E", [(1, 1, 1), (5, 2, 4), (600, 3, 8), (40000, 4, 128)])
 def test_plan_and_its_users_drop_copies_without_an_expert(dev, T, k, E):
     """Expert numbers below zero and past the last: no place for the copy, -1 behind the send order's last row, a zero
