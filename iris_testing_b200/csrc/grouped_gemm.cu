@@ -244,6 +244,16 @@ __host__ __device__ __forceinline__ bool fill_bucket(ControlSmem& c, const int* 
   return !(n > 0 && group_start + within + n > cap_rows) && n >= 0;
 }
 
+// Unit j of a bucket of `nrows` rows that starts at row `rel0` of the destination expert: its rows [p_lo, p_hi) of the
+// bucket, all in one aligned block of send_rows rows and so in one 128-row M-tile, whose counter the unit feeds.
+__host__ __device__ __forceinline__ void unit_rows(int rel0, int nrows, int j, int send_rows, int& tile, int& p_lo,
+                                                   int& p_hi) {
+  const int blk = rel0 / send_rows + j;
+  tile = blk * send_rows / BM;
+  p_lo = blk * send_rows > rel0 ? blk * send_rows - rel0 : 0;
+  p_hi = (blk + 1) * send_rows - rel0 < nrows ? (blk + 1) * send_rows - rel0 : nrows;
+}
+
 // Builds the sender tables and this rank's group sizes from the all-ranks
 // routing counts (`cnt` = counts_all[src][dst][e], staged in shared memory).  Runs on every
 // thread of the CTA.
@@ -889,10 +899,8 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a0,
         const int j = u - c.b_unit_start[bcur];
         const int rel0 = c.b_dst_rel0[bcur];
         const int nrows = c.b_count[bcur];
-        const int blk = rel0 / send_rows + j;    // aligned row block inside the destination expert
-        const int tile = blk * send_rows / BM;   // the 128-row M-tile whose counter it feeds
-        const int p_lo = max(0, blk * send_rows - rel0);
-        const int p_hi = min(nrows, (blk + 1) * send_rows - rel0);
+        int tile, p_lo, p_hi;
+        unit_rows(rel0, nrows, j, send_rows, tile, p_lo, p_hi);
         const int dst = c.b_dst_rank[bcur];
         const int send0 = c.b_send_start[bcur];
         const int drow0 = c.b_dst_row[bcur];
@@ -1244,17 +1252,19 @@ extern "C" int b200_debug_tile_walk(int total, int schedulers, int* owner) {
   return 0;
 }
 
-// tables: [7][world * e_local] = count, send_start, dst_row, dst_rel0, dst_mtile0, dst_rank, units
-extern "C" int b200_debug_dispatch_tables(const int* counts_all, int world, int e_local, int rank,
-                                          int cap_rows, int* g_rows, int* tables) {
+// tables: [7][world * e_local] = count, send_start, dst_row, dst_rel0, dst_mtile0, dst_rank, units of send_rows rows
+extern "C" int b200_debug_dispatch_tables_of(const int* counts_all, int world, int e_local, int rank,
+                                             int cap_rows, int send_rows, int* g_rows, int* tables) {
   using namespace b200;
   const int ET = world * e_local;
-  if (world < 1 || world > B200_MAX_WORLD || ET > B200_MAX_EXPERTS || rank < 0 || rank >= world) return -1;
+  if (world < 1 || world > B200_MAX_WORLD || ET > B200_MAX_EXPERTS || rank < 0 || rank >= world ||
+      (send_rows != SEND_ROWS && send_rows != SEND_ROWS_SHORT))
+    return -1;
   ControlSmem* c = new ControlSmem();
   int ok = 1;
   for (int e = 0; e < e_local; ++e) g_rows[e] = received_rows(counts_all, world, e_local, rank, e);
   for (int bi = 0; bi < ET; ++bi) {
-    if (!fill_bucket(*c, counts_all, world, e_local, rank, bi, cap_rows, SEND_ROWS)) ok = 0;
+    if (!fill_bucket(*c, counts_all, world, e_local, rank, bi, cap_rows, send_rows)) ok = 0;
     tables[0 * ET + bi] = c->b_count[bi];
     tables[1 * ET + bi] = c->b_send_start[bi];
     tables[2 * ET + bi] = c->b_dst_row[bi];
@@ -1265,4 +1275,14 @@ extern "C" int b200_debug_dispatch_tables(const int* counts_all, int world, int 
   }
   delete c;
   return ok;
+}
+
+extern "C" int b200_debug_dispatch_tables(const int* counts_all, int world, int e_local, int rank,
+                                          int cap_rows, int* g_rows, int* tables) {
+  return b200_debug_dispatch_tables_of(counts_all, world, e_local, rank, cap_rows, b200::SEND_ROWS, g_rows, tables);
+}
+
+// out: [units][3] = M-tile, first and past-last row of each unit of one bucket (as unit_rows gives them)
+extern "C" void b200_debug_unit_rows(int rel0, int nrows, int units, int send_rows, int* out) {
+  for (int j = 0; j < units; ++j) b200::unit_rows(rel0, nrows, j, send_rows, out[3 * j], out[3 * j + 1], out[3 * j + 2]);
 }

@@ -6,9 +6,10 @@
 // a serving loop that pre-sized all of its memory, under a framework whose
 // allocator must not be re-entered (a custom-op callback, a memory-pool hook),
 // or in a process that hands this library raw buffers and has no allocator to
-// offer for temporaries.  The regular entry point, b200_plan, needs a
-// caller-provided temporary (one int per routed copy, `rank_in_bucket`); here
-// that temporary lives in a fixed array inside the library instead.
+// offer for temporaries.  b200_plan_ws, which make_plan and the layer call, and
+// b200_plan need caller-provided temporaries (one int per routed copy,
+// `rank_in_bucket`; the former also a workspace); here that temporary lives in a
+// fixed array inside the library instead.
 //
 // What it does: the same two kernels as b200_plan.  From topk_idx (n_flat
 // global expert ids, token-major then slot) it writes

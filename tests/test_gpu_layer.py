@@ -369,6 +369,28 @@ def test_slot_reduction_splits_rows_over_warps(D, k, T):
     _finish(layer)
 
 
+@pytest.mark.parametrize("T,gated", [(300, True), (2400, True), (300, False), (2400, False)])
+def test_layers_in_a_row_without_a_synchronisation(T, gated):
+    """One layer's output is the next one's input while the kernels of both are chained: the router (one launch up to
+    4096 copies, three above) starts before the slot reduction it reads from has ended."""
+    from iris_testing_b200.config import MoEConfig
+    from iris_testing_b200.utils import gen_local_tokens
+    cfg = MoEConfig(hidden_dim=512, ffn_dim=256 if gated else 0, num_experts=8, topk=2, gated=gated)
+    (a, ha), (b, _) = _make(cfg, T, seed=1), _make(cfg, T, seed=2)
+    xs = [gen_local_tokens(1, T, 512, torch.bfloat16, ha.device, i, 0, "normal") for i in range(10)]
+    torch.cuda.synchronize()
+    mids, ends = [], []
+    for x in xs:
+        mids.append(a(x))
+        ends.append(b(mids[-1]))
+    for x, m, y in zip(xs, mids, ends):
+        _close(a, x, m)
+        assert torch.equal(y, b(m))                  # the same call with its input long settled
+        _close(b, m, y)
+    _finish(a)
+    _finish(b)
+
+
 @pytest.mark.parametrize("rows", [127, 128, 256, 257, 352, 353])
 def test_tile_geometry_follows_the_rows_of_each_call(rows):
     """Both sides of the lines between single CTAs and CTA pairs, in one layer made for more tokens."""

@@ -78,30 +78,32 @@ def test_even_rounds_tile_walk_covers_every_tile_in_the_minimum_number_of_rounds
     assert max(owner) == 127
 
 
-def dispatch_tables(lib, counts, W, EL, rank, cap):
+def dispatch_tables(lib, counts, W, EL, rank, cap, send_rows=32):
     ET = W * EL
     flat = [counts[s][d][e] for s in range(W) for d in range(W) for e in range(EL)]
     arr = (C.c_int * len(flat))(*flat)
     g_rows = (C.c_int * EL)()
     tables = (C.c_int * (7 * ET))()
-    ok = lib.b200_debug_dispatch_tables(arr, W, EL, rank, cap, g_rows, tables)
+    ok = lib.b200_debug_dispatch_tables_of(arr, W, EL, rank, cap, send_rows, g_rows, tables)
     t = [[tables[k * ET + b] for b in range(ET)] for k in range(7)]
     return ok, list(g_rows), dict(count=t[0], send_start=t[1], dst_row=t[2], rel0=t[3], mtile0=t[4],
                                   dst_rank=t[5], units=t[6])
 
 
+@pytest.mark.parametrize("send_rows", [8, 32])
 @pytest.mark.parametrize("W,EL", [(1, 8), (2, 4), (4, 2), (8, 1), (8, 16), (4, 32), (1, 128)])
-def test_cross_rank_row_layout_is_a_partition(W, EL):
+def test_cross_rank_row_layout_is_a_partition(W, EL, send_rows):
     """For every destination rank and expert, the row ranges that the sources compute for
     themselves tile that expert's block exactly, in the order self, self-1, self-2, ...;
-    send offsets follow the packed (destination, expert) order of the sender."""
+    send offsets follow the packed (destination, expert) order of the sender.  The sender's units (8 rows for
+    short batches, 32 otherwise) cut each bucket into its rows, none across an M-tile."""
     lib = _lib()
     rng = random.Random(W * 1000 + EL)
     for trial in range(6):
         counts = [[[rng.choice([0, 0, 1, 31, 32, 33, 127, 128, 300, rng.randint(0, 700)]) for _ in range(EL)]
                    for _ in range(W)] for _ in range(W)]
         cap = 1 << 24
-        per_rank = [dispatch_tables(lib, counts, W, EL, r, cap) for r in range(W)]
+        per_rank = [dispatch_tables(lib, counts, W, EL, r, cap, send_rows) for r in range(W)]
         for dst in range(W):
             rows_e = [sum(counts[s][dst][e] for s in range(W)) for e in range(EL)]
             assert per_rank[dst][1] == rows_e                      # receiver's view of its groups
@@ -119,8 +121,16 @@ def test_cross_rank_row_layout_is_a_partition(W, EL):
                     assert t["mtile0"][bi] == mtile0[e]
                     n = counts[src][dst][e]
                     rel0 = t["rel0"][bi]
-                    units = ((rel0 + n - 1) // 32 - rel0 // 32 + 1) if n else 0
+                    units = ((rel0 + n - 1) // send_rows - rel0 // send_rows + 1) if n else 0
                     assert t["units"][bi] == units
+                    out = (C.c_int * (3 * max(units, 1)))()
+                    lib.b200_debug_unit_rows(rel0, n, units, send_rows, out)
+                    at = 0
+                    for j in range(units):
+                        tile, lo, hi = out[3 * j:3 * j + 3]
+                        assert lo == at and lo < hi and (rel0 + lo) // 128 == tile == (rel0 + hi - 1) // 128
+                        at = hi
+                    assert at == n
                     expect_row += n
                 assert expect_row == group_start[e] + rows_e[e]
         for src in range(W):                                        # packed send order of the sender

@@ -5,8 +5,9 @@ with all memory pre-sized, a callback running under a framework allocator that m
 be re-entered, a host program that only hands over raw buffers).  ``b200_plan_noalloc``
 gives them the dispatch plan with its temporary held in a fixed array inside the library.
 This test calls it twice in a row through ``ctypes`` and checks every output against the
-regular entry point ``b200_plan``; the second call uses different routing so that stale
-contents of the shared array would show.  It lives in a file that pytest collects last.
+entry point with a caller's temporary, ``b200_plan``; the second call uses different routing so that stale
+contents of the shared array would show, and ``make_plan`` (whose kernels read the list once) has to give the
+same.  It lives in a file that pytest collects last.
 """
 import ctypes as C
 
@@ -31,6 +32,7 @@ def _regular(lib, idx, E, stream):
 
 def test_plan_noalloc_matches_regular_entry_point_twice():
     from iris_testing_b200 import _native
+    from iris_testing_b200.ops import make_plan
     lib = _native.lib()
     fn = lib.b200_plan_noalloc
     fn.argtypes = [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
@@ -57,6 +59,9 @@ def test_plan_noalloc_matches_regular_entry_point_twice():
         torch.cuda.synchronize()
         assert torch.equal(counts, r_counts) and torch.equal(start, r_start)
         assert torch.equal(order, r_order) and torch.equal(slot, r_slot)
+        p = make_plan(idx, E)
+        assert torch.equal(counts, p.counts) and torch.equal(start, p.bucket_start)
+        assert torch.equal(order, p.send_order) and torch.equal(slot, p.dst_slot)
     # dst_slot is optional: without it the other outputs are unchanged
     order2 = torch.empty(n, **i32)
     assert fn(idx.data_ptr(), n, E, counts.data_ptr(), start.data_ptr(), order2.data_ptr(), None, stream) == 0
