@@ -366,14 +366,18 @@ class MoELayer(nn.Module):
         raise AssertionError("unreachable")
 
     SMALL_MAX_FLAT = 4096          # routed copies the single-launch route+plan kernel takes
-    SMALL_MAX_TRIPS = 16           # size of the routing work up to which one launch is taken (below)
+    SMALL_MAX_TRIPS = 16           # units of routing work up to which one launch is taken (below)
 
     def uses_small_path(self, T: int) -> bool:
         """True when a forward of ``T`` tokens takes the small-token path: router and plan in ONE
-        launch instead of three.  At most 4096 routed copies (the plan is made by one CTA), and at most
-        16 units of eight experts x 512 columns per token and 1184 tokens: beyond that the separate kernels
-        spread the work better.  Mixtral shape, one launch against three: 10 / 19 us at 64 tokens,
-        16 / 22 us at 2048."""
+        launch instead of three.  At most 4096 routed copies, since one CTA makes the plan from registers, and at
+        most 16 units of work (eight experts x 512 columns for 1184 tokens).
+
+        The second line does not lie where the two forms are equal: the one launch was faster at every point measured
+        (one / three launches, us: 4096 columns, 8 experts 7 / 30 at 64 tokens, 9 / 33 at 1185, 10 / 33 at 2048; 2048
+        columns, 32 experts 13 / 26 at 1000; and beyond the line 6144 columns, 8 experts 11 / 45 at 1729, 2048 columns, 64
+        experts, top-8 15 / 33 at 200).  It says which batches have which router: the two sum in different orders,
+        so moving it would route near-ties of those batches otherwise."""
         cfg = self.cfg
         if not self.small_path or T * cfg.topk > self.SMALL_MAX_FLAT:
             return False

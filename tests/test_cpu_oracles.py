@@ -241,7 +241,7 @@ def test_zero_padding_clears_stale_rows_only():
 
 def test_small_token_path_rule():
     """Which batches take the one-launch router + plan: at most 4096 routed copies and at most 16
-    load trips per router warp (decided on the host from the shape alone)."""
+    units of eight experts x 512 columns for 1184 tokens (decided on the host from the shape alone)."""
     from iris_testing_b200.config import MoEConfig
     from iris_testing_b200.models import MoELayer
 
