@@ -35,7 +35,9 @@ def pairs_pay(rows: float) -> bool:
     128, 821 / 672 at 160, 813 / 670 at 225).  Just above 256 rows most groups would fill a
     second 256-row tile by less than half, and three 128-row tiles are less padding (1093 / 1164 us at
     275 rows, 1131 / 1207 at 300, 1148 / 1275 at 350; 64 fine-grained experts 562 / 574 at 300); towards 384 that
-    is used up (589 / 589, one Linear 568 / 540) and from 512 on pairs win again (1575 / 1513)."""
+    is used up (589 / 589, one Linear 568 / 540) and from 512 on pairs win again (1575 / 1513).
+    Only the average is known here: at 250 rows half of the experts lie above 256, and pairs still win (785 - 997 /
+    756 - 949 over three routings)."""
     return rows >= 128 and not 256 < rows <= 352
 
 
